@@ -3,6 +3,7 @@
 #pragma once
 #include "hm_ctx.h"
 #include "sre_kernels.cuh"
+#include "sre_wide.cuh"
 #include "sweep3.cuh"
 
 namespace hm {
@@ -81,6 +82,30 @@ static int launch_fused(hm_ctx *c, const SreArgs &a0, int *nwarps_out) {
                     sizeof(double) * 2 * (QSet<QS>::NQ + 1) * (size_t)nwarps));
   a.partials = c->d_partials;
   kern<<<(unsigned)blocks, FUSED_WARPS * 32, smem, c->stream>>>(a);
+  c->launches += 1;
+  HM_CUDA(c, cudaGetLastError());
+  *nwarps_out = nwarps;
+  return HM_OK;
+}
+
+// n = 12, 13, 14: one CTA of G = 2^(n-11) warps per X-string (see k_sre_wide).  n = 14 is
+// the last size whose planes (128 KB in FP64) and registers (8 warps of 255) fit an SM; the
+// two-pass sweep was half as fast at each of the three sizes (figures in sre_wide.cuh).
+template <typename T, int G, int QS>
+static int launch_wide(hm_ctx *c, const SreArgs &a0, int *nwarps_out) {
+  SreArgs a = a0;
+  const size_t smem = (size_t)2048 * G * sizeof(T);
+  auto kern = k_sre_wide<T, G, QS>;
+  HM_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int occ = 0;
+  HM_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 32 * G, smem));
+  if (occ < 1) occ = 1;
+  const uint64_t blocks = std::min<uint64_t>(a.k_end - a.k_begin, (uint64_t)c->num_sms * occ);
+  const int nwarps = (int)blocks * G;
+  HM_TRY(ensure_dev(c, (void **)&c->d_partials, &c->partials_cap,
+                    sizeof(double) * 2 * (QSet<QS>::NQ + 1) * (size_t)nwarps));
+  a.partials = c->d_partials;
+  kern<<<(unsigned)blocks, 32 * G, smem, c->stream>>>(a);
   c->launches += 1;
   HM_CUDA(c, cudaGetLastError());
   *nwarps_out = nwarps;
@@ -313,9 +338,12 @@ static int dispatch_sre(hm_ctx *c, const SreArgs &a, int *nw) {
     }
   } else {
     switch (nb - PB) {
-      HM_2P_CASE(1)
-      HM_2P_CASE(2)
-      HM_2P_CASE(3)
+      case 1:
+        return launch_wide<T, 2, QS>(c, a, nw);
+      case 2:
+        return launch_wide<T, 4, QS>(c, a, nw);
+      case 3:
+        return launch_wide<T, 8, QS>(c, a, nw);
       HM_2P_CASE(4)
       HM_2P_CASE(5)
       HM_2P_CASE(6)

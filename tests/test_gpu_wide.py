@@ -1,0 +1,33 @@
+"""The sweep kernels of csrc/sre_wide.cuh against the queue sweep, which transforms the same
+X-strings by the two-pass route: sub-ranges of the Gray codes that are ragged, start past 0
+or hold a single X-string, every moment set, both precisions.
+
+FP64 sums are added from different operation orders of ~20 roundings per value; the
+averaging over 2^n values keeps the difference near 1e-16, 1e-13 is the bound used between
+the engines elsewhere.  FP32 is held to the precision's stated 1e-6."""
+import pytest
+
+from conftest import rand_state
+
+pytestmark = pytest.mark.gpu
+
+QS = {"q2": (2.0,), "q23": (2.0, 3.0), "gen": (4.0, 2.5, 1.0)}
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("qs", sorted(QS))
+@pytest.mark.parametrize("n", [12, 13, 14])
+def test_single_cta_ranges(ctx, hm, n, qs, precision):
+    N = hm._native
+    psi = rand_state(1 << n, 900 + n)
+    full = 1 << n
+    tol = 1e-13 if precision == "fp64" else 1e-6
+    for kb, ke in [(0, 1), (0, 150), (1, 2), (700, 1333), (full - 37, full)]:
+        p2, m = ctx.sre_range(psi, kb, ke, QS[qs], hm.PRECISIONS[precision])
+        try:
+            N.set_param(N.HM_PARAM_ENGINE, 2)
+            p2r, mr = ctx.sre_range(psi, kb, ke, QS[qs], hm.PRECISIONS[precision])
+        finally:
+            N.set_param(N.HM_PARAM_ENGINE, 0)
+        assert p2.sum() == pytest.approx(p2r.sum(), rel=tol)
+        assert m.sum(axis=1) == pytest.approx(mr.sum(axis=1), rel=tol)
