@@ -9,23 +9,30 @@
 namespace hm {
 
 // Tunables of the two-pass stage kernels (set through hm_set_param): a batch holds about
-// `units_target` warp units per pass (X = units_target / 2^HI X-strings, or X when set
+// `units_target` warp units per pass (X = units_target / 2^(n-11) X-strings, or X when set
 // explicitly), the two-batch ring stays within `ring_mib`, and `graph_stages` stages are
-// captured per CUDA graph.  Every stage costs a fixed few microseconds (launch, the first
-// loads of all warps at once, the tail), which favours large batches, while a ring that
-// outgrows the 126 MB L2 costs DRAM traffic.  Where they pull apart (n >= 18) the default
-// batch comes from `measured_x`, timed on B200 (us per X-string, stage kernels chained
-// by programmatic dependent launch, dead tiles discarded):
-//   FP64  n = 18: X = 32 (0.95; X = 24 1.01)  n = 19: X = 16 (1.89; X = 12 1.91, X = 4 1.94)
-//         n = 20: X = 10 (3.86; X = 8 4.05, X = 12 3.91, X = 16 4.18)  n = 21: X = 2 (10.6; X = 3 14.5)
-//   FP32  n = 18: X = 64 (0.49)  n = 19: X = 32 (1.02; X = 16 1.09)
-//         n = 20: X = 8 (2.72; X = 10 2.74, X = 12 3.06)  n = 21: X = 2 (10.4; X = 4 11.2)
-// Any X works (the kernel decodes units with a division); larger rings than the L2 can
-// still win while the stage count falls.  hm_autotune measures and records a batch for the
-// machine at hand; setting HM_PARAM_BATCH, _UNITS or _RING switches to the generic rule.
+// captured per CUDA graph.  A stage costs about 1.4 us beyond its rounds of items over the
+// groups of warps, and a last round that is not full costs a whole one; the ring's size
+// costs DRAM traffic once it outgrows the 126 MB L2.  The default batch `measured_x` is the
+// best of those that give whole rounds (2 X 2^HI items over 592 groups of two warps:
+// X = 37 m at n = 17) within a ring of about 120 MiB, timed on B200 (us per X-string):
+//   FP64  n = 15: X = 148 (0.107; 74: 0.120)    n = 16: X = 111 (0.191; 74: 0.195, 37: 0.22)
+//         n = 17: X = 55 (0.377; 37: 0.387)     n = 18: X = 27 (0.784; 18: 0.785, 37: 0.796)
+//         n = 19: X = 9 (1.735; 14: 1.759, 4: 1.83)  n = 21: X = 2 (9.40; 3: 9.68)
+//   FP32  n = 15: X = 296 (0.062; 256: 0.070)  n = 16: X = 148 (0.106; 74: 0.124)
+//         n = 17: X = 110 (0.197; 74: 0.204)    n = 18: X = 55 (0.403; 37: 0.413)
+//         n = 19: X = 18 (0.861; 28: 0.878)     n = 20: X = 9 (1.97; 7: 2.02)
+//         n = 21: X = 4 (4.65; 2: 4.90)
+// Against the rows and tiles of k_sre_stage, which ran every size before: FP64 0.116, 0.206,
+// 0.430, 0.852, 1.815, 3.79, 10.33 for n = 15 .. 21, FP32 0.067, 0.115, 0.221, 0.446, 0.967,
+// 2.70, 10.02.  FP64 at n = 20 stays with k_sre_stage (X = 10: 3.79; 3.87 here at X = 7):
+// both are bound by the ring's traffic there, and its tensor stores need no group of four.
+// So does FP64 at n = 19 for q = 2 and 3 together (X = 16: 1.88; 1.91 here).
+// hm_autotune measures and records a batch for the machine at hand; setting
+// HM_PARAM_BATCH, _UNITS or _RING switches to the generic rule.
 inline int measured_x(bool fp64, int n) {
-  static const int f64[4] = {32, 16, 10, 2}, f32[4] = {64, 32, 8, 2};
-  return (n >= 18 && n <= 21) ? (fp64 ? f64 : f32)[n - 18] : 0;
+  static const int f64[7] = {148, 111, 55, 27, 9, 10, 2}, f32[7] = {296, 148, 110, 55, 18, 9, 4};
+  return (n >= 15 && n <= 21) ? (fp64 ? f64 : f32)[n - 15] : 0;
 }
 
 struct TwoPassCfg {
@@ -118,13 +125,13 @@ static int launch_wide(hm_ctx *c, const SreArgs &a0, int *nwarps_out) {
 // sweeps replay a captured graph of G stages, with a one-thread kernel advancing the stage
 // base in device memory after every replay.
 template <typename Kern, typename Args>
-static int run_stage_chain(hm_ctx *c, Kern kern, Args &a, int nst, int blocks, size_t smem, int G,
+static int run_stage_chain(hm_ctx *c, Kern kern, Args &a, int nst, int blocks, int threads, size_t smem, int G,
                            const char *what) {
   auto launch = [&](int s) {
     a.node = s;
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3(blocks);
-    lc.blockDim = dim3(SRE_WARPS * 32);
+    lc.blockDim = dim3(threads);
     lc.dynamicSmemBytes = smem;
     lc.stream = c->stream;
     cudaLaunchAttribute at[1];
@@ -190,7 +197,7 @@ static int launch_stages(hm_ctx *c, const SreArgs &a0, int *nwarps_out) {
   const bool generic = cfg.X_set || cfg.units_target != def.units_target || cfg.ring_mib != def.ring_mib;
   uint64_t X, ring_mib = (uint64_t)cfg.ring_mib;
   const int tuned = cfg.tuned_x[sizeof(T) == 8 ? 0 : 1][a.n];
-  const int measured = generic ? 0 : measured_x(sizeof(T) == 8, a.n);
+  const int measured = generic ? 0 : (a.n == 19 ? 16 : measured_x(sizeof(T) == 8, a.n));
   if (cfg.X_set) {
     X = (uint64_t)cfg.X;
   } else if (tuned > 0 || measured > 0) {
@@ -239,7 +246,67 @@ static int launch_stages(hm_ctx *c, const SreArgs &a0, int *nwarps_out) {
   HM_CUDA(c, cudaMemsetAsync(c->d_ctrl, 0, 4 * sizeof(unsigned), c->stream));
   a.stage = c->d_ctrl;
   const int nst = a.nbatch + 1;
-  HM_TRY(run_stage_chain(c, kern, a, nst, blocks, smem, cfg.graph_stages, "stage"));
+  HM_TRY(run_stage_chain(c, kern, a, nst, blocks, SRE_WARPS * 32, smem, cfg.graph_stages, "stage"));
+  *nwarps_out = nwarps;
+  return HM_OK;
+}
+
+// Warps per pass-1 group of the two-pass sweep at n qubits: two (rows of 2048 complex
+// values), more from the size on where pass 2 would otherwise hold more than one row bit on
+// lane bits and read less than 128 bytes per row and unit, whole lines that it can discard
+// (FP32 at n = 19: 0.861 us per X-string with four, 0.966 with two).
+template <typename T> constexpr int wide_group(int n) {
+  return n <= (sizeof(T) == 8 ? 19 : 18) ? 2 : n <= 20 ? 4 : 8;
+}
+
+// Two-pass sweep (see k_sre_wide_stage): ring of two batches, stages chained and replayed
+// from a captured CUDA graph.
+template <typename T, int N, int QS>
+static int launch_wide_stages(hm_ctx *c, const SreArgs &a0, int *nwarps_out) {
+  constexpr int G = wide_group<T>(N), HI = N - 11 - ilog2c(G), NQ = QSet<QS>::NQ, WARPS = WideCta<G>::WARPS;
+  const TwoPassCfg cfg = twopass_cfg();
+  WideArgs a;
+  memset(&a, 0, sizeof a);
+  a.psi = a0.psi;
+  a.k_begin = a0.k_begin;
+  a.k_end = a0.k_end;
+  a.qp = a0.qp;
+  const uint64_t len = a.k_end - a.k_begin, per_x = ((uint64_t)1 << N) * sizeof(T);
+  const TwoPassCfg def;
+  const bool generic = cfg.X_set || cfg.units_target != def.units_target || cfg.ring_mib != def.ring_mib;
+  uint64_t X, ring_mib = (uint64_t)cfg.ring_mib;
+  const int tuned = cfg.tuned_x[sizeof(T) == 8 ? 0 : 1][N];
+  const int measured = generic ? 0 : measured_x(sizeof(T) == 8, N);
+  if (cfg.X_set) {
+    X = (uint64_t)cfg.X;
+  } else if (tuned > 0 || measured > 0) {
+    X = (uint64_t)(tuned > 0 ? tuned : measured);
+    ring_mib = std::max<uint64_t>(ring_mib, (2 * X * per_x + (1 << 20) - 1) >> 20);
+  } else {
+    X = std::max<uint64_t>(1, (uint64_t)cfg.units_target >> (N - 11));
+  }
+  while (X > 1 && 2 * X * per_x > (ring_mib << 20)) X >>= 1;
+  if (X > len) X = len;
+  a.X = (int)X;
+  a.nbatch = (int)((len + X - 1) / X);
+  HM_TRY(ensure_dev(c, &c->d_inter, &c->inter_cap, 2 * (size_t)X * per_x));
+  a.ring = c->d_inter;
+  const size_t smem = (size_t)WARPS * 2048 * sizeof(T);
+  auto kern = k_sre_wide_stage<T, G, HI, QS>;
+  HM_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int occ = 0;
+  HM_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, WARPS * 32, smem));
+  if (occ < 1) occ = 1;
+  const long long items = 2 * (long long)X << HI;
+  const int blocks = (int)std::min<long long>((long long)c->num_sms * occ, (items * G + WARPS - 1) / WARPS);
+  const int nwarps = blocks * WARPS;
+  HM_TRY(ensure_dev(c, (void **)&c->d_partials, &c->partials_cap, sizeof(double) * 2 * (NQ + 1) * (size_t)nwarps));
+  HM_CUDA(c, cudaMemsetAsync(c->d_partials, 0, sizeof(double) * 2 * (NQ + 1) * (size_t)nwarps, c->stream));
+  a.slots = c->d_partials;
+  HM_TRY(ensure_dev(c, (void **)&c->d_ctrl, &c->ctrl_cap, 4 * sizeof(unsigned)));
+  HM_CUDA(c, cudaMemsetAsync(c->d_ctrl, 0, 4 * sizeof(unsigned), c->stream));
+  a.stage = c->d_ctrl;
+  HM_TRY(run_stage_chain(c, kern, a, a.nbatch + 1, blocks, WARPS * 32, smem, cfg.graph_stages, "stage"));
   *nwarps_out = nwarps;
   return HM_OK;
 }
@@ -303,7 +370,7 @@ static int launch_stages3(hm_ctx *c, const SreArgs &a0, int *nwarps_out) {
   HM_CUDA(c, cudaMemsetAsync(c->d_ctrl, 0, 4 * sizeof(unsigned), c->stream));
   a.stage = c->d_ctrl;
   const int nst = a.nbatch + 2;
-  HM_TRY(run_stage_chain(c, kern, a, nst, blocks, smem, cfg.graph_stages, "three-pass"));
+  HM_TRY(run_stage_chain(c, kern, a, nst, blocks, SRE_WARPS * 32, smem, cfg.graph_stages, "three-pass"));
   *nwarps_out = nwarps;
   return HM_OK;
 }
@@ -311,10 +378,6 @@ static int launch_stages3(hm_ctx *c, const SreArgs &a0, int *nwarps_out) {
 #define HM_FUSED_CASE(NBv)                                         \
   case NBv:                                                        \
     return launch_fused<T, R, ((NBv) <= PB ? (NBv) : PB), QS>(c, a, nw);
-#define HM_2P_CASE(HIv)                                            \
-  case HIv:                                                        \
-    return launch_stages<T, R, ((HIv) <= PB ? (HIv) : PB), QS>(c, a, nw);
-
 template <typename T, int R, int QS>
 static int dispatch_sre(hm_ctx *c, const SreArgs &a, int *nw) {
   constexpr int PB = ilog2c(R) + 5;
@@ -344,13 +407,26 @@ static int dispatch_sre(hm_ctx *c, const SreArgs &a, int *nw) {
         return launch_wide<T, 4, QS>(c, a, nw);
       case 3:
         return launch_wide<T, 8, QS>(c, a, nw);
-      HM_2P_CASE(4)
-      HM_2P_CASE(5)
-      HM_2P_CASE(6)
-      HM_2P_CASE(7)
-      HM_2P_CASE(8)
-      HM_2P_CASE(9)
-      HM_2P_CASE(10)
+      case 4:
+        return launch_wide_stages<T, 15, QS>(c, a, nw);
+      case 5:
+        return launch_wide_stages<T, 16, QS>(c, a, nw);
+      case 6:
+        return launch_wide_stages<T, 17, QS>(c, a, nw);
+      case 7:
+        return launch_wide_stages<T, 18, QS>(c, a, nw);
+      case 8:  // FP64, q = 2 and 3: see measured_x
+        if constexpr (sizeof(T) == 8 && QS == QS_Q23)
+          return launch_stages<T, R, 8, QS>(c, a, nw);
+        else
+          return launch_wide_stages<T, 19, QS>(c, a, nw);
+      case 9:  // FP64, q = 2 (and 3): see measured_x
+        if constexpr (sizeof(T) == 8 && QS != QS_GEN)
+          return launch_stages<T, R, 9, QS>(c, a, nw);
+        else
+          return launch_wide_stages<T, 20, QS>(c, a, nw);
+      case 10:
+        return launch_wide_stages<T, 21, QS>(c, a, nw);
       case 11:
         if constexpr (R == 32) return launch_stages3<T, R, 1, QS>(c, a, nw);
         break;
@@ -380,5 +456,17 @@ int launch_sre_qs(hm_ctx *c, const void *psi_dev, int n, uint64_t kb, uint64_t k
   a.qp = qp;
   return dispatch_sre<T, R, QS>(c, a, nwarps);
 }
+
+// one translation unit per precision and moment set holds the kernels (sre_fp64_q2.cu, ...)
+#define HM_EXTERN_SRE(T, QS)                                                                             \
+  extern template int launch_sre_qs<T, 32, QS>(hm_ctx *, const void *, int, uint64_t, uint64_t,          \
+                                               const QParams &, int *);
+HM_EXTERN_SRE(double, QS_Q2)
+HM_EXTERN_SRE(double, QS_Q23)
+HM_EXTERN_SRE(double, QS_GEN)
+HM_EXTERN_SRE(float, QS_Q2)
+HM_EXTERN_SRE(float, QS_Q23)
+HM_EXTERN_SRE(float, QS_GEN)
+#undef HM_EXTERN_SRE
 
 }  // namespace hm

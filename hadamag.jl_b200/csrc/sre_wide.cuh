@@ -24,6 +24,40 @@
 
 namespace hm {
 
+// One butterfly of registers i and i | 1 << S.
+template <int S, typename V>
+__device__ __forceinline__ void bfly(V (&v)[32], int i) {
+  const int k = i | (1 << S);
+  const V a = v[i], b = v[k];
+  v[i] = v_add(a, b);
+  v[k] = v_sub(a, b);
+}
+// The 32-register transforms run as 4 x 8: index bits 0, 1 inside each block of four
+// registers (as soon as the block has arrived), then bits 2 .. 4 inside each of the four
+// classes i mod 4 (each leaves as soon as it is done), so that the loads and stores of one
+// part overlap the arithmetic of another.
+template <int LO, int HI, typename V>
+__device__ __forceinline__ void wht_block(V (&v)[32], int b) {
+#pragma unroll
+  for (int i = 4 * b; i < 4 * b + 4; ++i)
+    if (LO <= 0 && HI > 0 && !(i & 1)) bfly<0>(v, i);
+#pragma unroll
+  for (int i = 4 * b; i < 4 * b + 4; ++i)
+    if (LO <= 1 && HI > 1 && !(i & 2)) bfly<1>(v, i);
+}
+template <int LO, int HI, typename V>
+__device__ __forceinline__ void wht_class(V (&v)[32], int c) {
+#pragma unroll
+  for (int i = c; i < 32; i += 4)
+    if (LO <= 2 && HI > 2 && !(i & 4)) bfly<2>(v, i);
+#pragma unroll
+  for (int i = c; i < 32; i += 4)
+    if (LO <= 3 && HI > 3 && !(i & 8)) bfly<3>(v, i);
+#pragma unroll
+  for (int i = c; i < 32; i += 4)
+    if (LO <= 4 && HI > 4 && !(i & 16)) bfly<4>(v, i);
+}
+
 // threads of one group meet (id 0 .. 15; the group's warps are whole warps)
 template <int NT>
 __device__ __forceinline__ void group_sync(int id) {
@@ -41,12 +75,16 @@ __device__ __forceinline__ uint32_t wide_pos(uint32_t e) {
 
 // phase A's 32 complex registers -> the two planes
 template <typename T, int G, typename V>
-__device__ __forceinline__ void wide_put(const V (&v)[32], T *buf, int w, int lane) {
+__device__ __forceinline__ void wide_put(V (&v)[32], T *buf, int w, int lane) {
 #pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    const uint32_t p = wide_pos<T>((uint32_t)(32 * i + lane)) + 1024u * w;
-    buf[p] = v[i].x;
-    buf[1024 * G + p] = v[i].y;
+  for (int c = 0; c < 4; ++c) {
+    wht_class<2, 5>(v, c);
+#pragma unroll
+    for (int i = c; i < 32; i += 4) {
+      const uint32_t p = wide_pos<T>((uint32_t)(32 * i + lane)) + 1024u * w;
+      buf[p] = v[i].x;
+      buf[1024 * G + p] = v[i].y;
+    }
   }
 }
 
@@ -153,36 +191,56 @@ __device__ __noinline__ void wide_moments_gen(const T *sm, int lane, double *s, 
   for (int t = 0; t < 4; ++t) s[1 + t] = ag[t];
 }
 
-// Butterflies of phase B's register bits and the per-lane sums of F^2 and (F^2)^q.
+// Butterflies over the LV low bits of the register index (and, with PAIR, over the bit inside
+// a pair), then the per-lane sums of F^2 and (F^2)^q.
 // q = 2 alone: the last two bits are not transformed.  For four values u_e before them,
 // with c_d = sum_e u_e u_(e^d), the four outputs satisfy sum F^2 = 4 c_0 and
 // sum F^4 = 4 (c_0^2 + c_1^2 + c_2^2 + c_3^2) (F_k^2 = sum_d (-1)^(k.d) c_d, Parseval over k):
 // 15 operations for the four values instead of 8 for the two bits and 12 for the powers.
-template <int QS, typename T, typename V>
+template <int QS, int LV, bool PAIR, typename T, typename V>
 __device__ __forceinline__ void wide_moments(V (&v)[32], double *s, const QParams &qp, T *sm, int lane) {
   if constexpr (QS == QS_Q2) {
-    reg_wht<32, 0, 4>(v);
-    double a2[2] = {0.0, 0.0}, m0[2] = {0.0, 0.0}, h1 = 0.0, h2 = 0.0, h3 = 0.0;
+    constexpr int TOP = PAIR ? LV - 1 : LV - 2;  // transformed explicitly: index bits 0 .. TOP-1
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const double u0 = v[i].x, u1 = v[i].y, u2 = v[i + 16].x, u3 = v[i + 16].y;
+    for (int b = 0; b < 8; ++b) wht_block<0, TOP>(v, b);
+    double a2[2] = {0.0, 0.0}, m0[2] = {0.0, 0.0}, h1 = 0.0, h2 = 0.0, h3 = 0.0;
+    auto quad = [&](int t, double u0, double u1, double u2, double u3) {
       const double c0 = fma(u0, u0, fma(u1, u1, fma(u2, u2, u3 * u3)));
       const double c1 = fma(u0, u1, u2 * u3), c2 = fma(u0, u2, u1 * u3), c3 = fma(u0, u3, u1 * u2);
-      a2[i & 1] += c0;
-      m0[i & 1] = fma(c0, c0, m0[i & 1]);
+      a2[t] += c0;
+      m0[t] = fma(c0, c0, m0[t]);
       h1 = fma(c1, c1, h1);
       h2 = fma(c2, c2, h2);
       h3 = fma(c3, c3, h3);
+    };
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      wht_class<0, TOP>(v, c);
+#pragma unroll
+    for (int i = TOP >= 2 ? c : 8 * c; i < (TOP >= 2 ? 32 : 8 * c + 8); i += (TOP >= 2 ? 4 : 1)) {
+      if constexpr (PAIR) {
+        if ((i >> TOP) & 1) continue;
+        const int k = i | (1 << TOP);
+        quad(i & 1, v[i].x, v[i].y, v[k].x, v[k].y);
+      } else {
+        if ((i >> TOP) & 3) continue;
+        const int k = i | (1 << TOP), m = i | (2 << TOP);
+        quad(0, v[i].x, v[k].x, v[m].x, v[m | k].x);
+        quad(1, v[i].y, v[k].y, v[m].y, v[m | k].y);
+      }
+    }
     }
     s[0] = 4.0 * (a2[0] + a2[1]);
     s[1] = 4.0 * ((m0[0] + m0[1]) + 4.0 * ((h1 + h2) + h3));
   } else {
-    reg_wht<32, 0, 5>(v);
+    reg_wht<32, 0, LV>(v);
+    if constexpr (PAIR) {
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      const auto a = v[i].x, b = v[i].y;
-      v[i].x = a + b;
-      v[i].y = a - b;
+      for (int i = 0; i < 32; ++i) {
+        const auto a = v[i].x, b = v[i].y;
+        v[i].x = a + b;
+        v[i].y = a - b;
+      }
     }
     if constexpr (QS == QS_GEN) {
 #pragma unroll
@@ -194,6 +252,47 @@ __device__ __forceinline__ void wide_moments(V (&v)[32], double *s, const QParam
     } else {
       lane_moments<32, QS>(v, s, qp, (V *)nullptr, lane);  // q = 2 and 3: no staging
     }
+  }
+}
+
+// Phase A of X-string x for element e0 + 32 i in register i (e0 includes the lane): products
+// and butterflies over bits 5 .. 9.  r(e) is e with a zero inserted at the highest set bit
+// of x, e + (the bits of e from there up), for any position of that bit; x = 0 pairs the
+// top bit (half = 2^(n-1)).
+template <typename V>
+__device__ __forceinline__ void wide_build(V (&v)[32], const V *__restrict__ psi, uint32_t x, uint32_t e0,
+                                           uint32_t half) {
+  if (x != 0) {
+    const uint32_t up = ~((1u << (31 - __clz((int)x))) - 1u);
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+#pragma unroll
+      for (int i = 4 * b; i < 4 * b + 4; ++i) {
+        const uint32_t e = e0 + 32u * i, r = e + (e & up);
+        v[i] = conj_mul(ld_psi(psi + r), ld_psi(psi + (r ^ x)));
+      }
+      wht_block<0, 2>(v, b);
+    }
+  } else {
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+#pragma unroll
+      for (int i = 4 * b; i < 4 * b + 4; ++i) {
+        const uint32_t e = e0 + 32u * i;
+        v[i] = zero_pair(ld_psi(psi + e), ld_psi(psi + e + half));
+      }
+      wht_block<0, 2>(v, b);
+    }
+  }
+}
+
+// the transform bits that phase B keeps on lane bits
+template <int G, typename V>
+__device__ __forceinline__ void wide_lane_bits(V (&v)[32], int lane) {
+  if constexpr (G == 4) lane_wht(v, lane, 16);
+  if constexpr (G == 8) {
+    lane_wht(v, lane, 8);
+    lane_wht(v, lane, 16);
   }
 }
 
@@ -216,34 +315,15 @@ __global__ void __launch_bounds__(32 * G, WideOcc<T, G>::value) k_sre_wide(SreAr
   for (uint64_t k = a.k_begin + blockIdx.x; k < a.k_end; k += gridDim.x) {
     const uint32_t x = (uint32_t)gray_code(k);
     V v[32];
-    if (x != 0) {
-      // r = e with a zero inserted at the highest set bit of x: e + (the bits from there up)
-      const uint32_t up = ~((1u << (31 - __clz((int)x))) - 1u);
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const uint32_t e = e0 + 32u * i, r = e + (e & up);
-        v[i] = conj_mul(ld_psi(psi + r), ld_psi(psi + (r ^ x)));
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const uint32_t e = e0 + 32u * i;
-        v[i] = zero_pair(ld_psi(psi + e), ld_psi(psi + e + (1u << NB)));
-      }
-    }
-    reg_wht<32, 0, 5>(v);  // element bits 5 .. 9
+    wide_build(v, psi, x, e0, 1u << NB);
     __syncthreads();       // the previous X-string's values have been read
     wide_put<T, G>(v, buf, w, lane);
     __syncthreads();
     wide_get<T, G>(v, buf, w, lane);
-    if constexpr (G == 4) lane_wht(v, lane, 16);
-    if constexpr (G == 8) {
-      lane_wht(v, lane, 8);
-      lane_wht(v, lane, 16);
-    }
+    wide_lane_bits<G>(v, lane);
     double s[NQ + 1];
     if constexpr (QS == QS_GEN) __syncthreads();  // the moments stage their values in the buffer
-    wide_moments<QS>(v, s, a.qp, buf + 2048 * w, lane);
+    wide_moments<QS, 5, true>(v, s, a.qp, buf + 2048 * w, lane);
     s[0] = x == 0 ? s[0] : 4.0 * s[0];
 #pragma unroll
     for (int t = 0; t < NQ; ++t) s[1 + t] *= q_scale<QS>(t, x == 0, a.qp);
@@ -262,6 +342,160 @@ __global__ void __launch_bounds__(32 * G, WideOcc<T, G>::value) k_sre_wide(SreAr
     }
   }
   if (lane == 0) write_partials<NQ>(a.partials, blockIdx.x * G + w, acc);
+}
+
+// ---------------------------------------------------------------------------------
+// Two-pass sweep for 15 <= n <= 21 as a sequence of stage kernels (chained and replayed as
+// k_sre_stage's: stage t runs pass 1 of batch t and pass 2 of batch t - 1, slot b & 1).
+//   pass 1  a group of G warps transforms the low 10 + log2 G bits of the (n-1)-bit index:
+//           phase A, exchange, phase B as above.  Its 2048 G real values leave straight from
+//           the registers as one row of the intermediate, pairs in register order (any
+//           fixed relabelling of the columns is invisible to the sums): whole 512-byte
+//           (FP64) or 256-byte stores, no staging.
+//   pass 2  columns of the 2^HI rows, HI = n - 11 - log2 G.  A lane holds 64 values; a warp
+//           2^HI rows of 2^(11-HI) columns.  HI <= 5: pairs of columns, up to 32 rows in
+//           registers.  HI >= 6: six row bits in registers, the others on lane bits.
+// No value crosses shared memory in pass 2.  L1-path bytes per complex element: 32 gather,
+// 32 exchange, 16 store, 16 load, 16 per lane bit, against 144 for rows and tiles of 1024
+// with an exchange in each pass and tensor stores.
+struct WideArgs {
+  const void *psi;
+  void *ring;       // 2 slots x X strings x 2^n values of T: rows of 2048 G
+  double *slots;    // per warp: 2 (1 + NQ) doubles
+  unsigned *stage;  // [0] stage index of node 0 of the current graph replay
+  uint64_t k_begin, k_end;
+  QParams qp;
+  int X, nbatch;
+  int node;         // position of this launch in the captured graph
+};
+
+template <int G> struct WideCta { static constexpr int WARPS = G < 4 ? 4 : G; };
+
+template <typename T, int G, int HI, int QS>
+__global__ void __launch_bounds__(32 * WideCta<G>::WARPS, (sizeof(T) == 8 ? 8 : 16) / WideCta<G>::WARPS)
+    k_sre_wide_stage(const __grid_constant__ WideArgs a) {
+  using V = typename VT<T>::V;
+  constexpr int NQ = QSet<QS>::NQ, NG = WideCta<G>::WARPS / G;  // groups per CTA
+  constexpr uint32_t ROW = 2048 * G, NROW = 1u << HI;
+  extern __shared__ __align__(128) unsigned char smem_wide[];
+  allow_next_grid();
+  // the base only changes between replays, after every node of the replay has finished
+  const long long t = (long long)*(volatile unsigned *)a.stage + a.node;
+  if (t > a.nbatch) return;  // padding stages of the last graph replay
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int grp = warp / G, w = warp % G;
+  T *buf = reinterpret_cast<T *>(smem_wide) + (size_t)grp * ROW;
+  const V *psi = reinterpret_cast<const V *>(a.psi);
+  T *ring = reinterpret_cast<T *>(a.ring);
+  const long long per = (long long)a.X * NROW;    // items (row or G column blocks) per pass
+  const long long n1 = t < a.nbatch ? per : 0;    // pass 1 of batch t
+  const long long n2 = t >= 1 ? per : 0;          // pass 2 of batch t - 1
+  const long long gid = (long long)blockIdx.x * NG + grp, ngrp = (long long)gridDim.x * NG;
+  dd acc[NQ + 1];
+#pragma unroll
+  for (int q = 0; q <= NQ; ++q) acc[q] = dd{0.0, 0.0};
+  const long long nfirst = n1 < ngrp ? n1 : ngrp;
+  for (long long u = gid; u < n1 + n2; u += ngrp) {
+    const bool p2 = u >= nfirst && u < nfirst + n2;
+    const long long r = p2 ? u - nfirst : (u < nfirst ? u : u - n2);
+    const long long b = p2 ? t - 1 : t;
+    const uint32_t xs = (uint32_t)(r % a.X), sub = (uint32_t)(r / a.X);
+    const uint64_t k = a.k_begin + (uint64_t)b * a.X + xs;
+    if (k >= a.k_end) continue;
+    const uint32_t x = (uint32_t)gray_code(k);
+    T *inter = ring + ((size_t)(b & 1) * a.X + xs) * ((size_t)NROW * ROW);
+    V v[32];
+    if (!p2) {
+      wide_build(v, psi, x, sub * (1024u * G) + 1024u * w + lane, NROW * (1024u * G));
+      group_sync<32 * G>(1 + grp);  // the group's previous values have been read
+      wide_put<T, G>(v, buf, w, lane);
+      group_sync<32 * G>(1 + grp);
+      wide_get<T, G>(v, buf, w, lane);
+      wide_lane_bits<G>(v, lane);
+#pragma unroll
+      for (int b = 0; b < 8; ++b) wht_block<0, 2>(v, b);
+      wait_prior_grid();  // the slot that the previous stage's pass 2 read
+      V *row = reinterpret_cast<V *>(inter + (size_t)sub * ROW) + 1024 * w + lane;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        wht_class<2, 5>(v, c);
+#pragma unroll
+        for (int i = c; i < 32; i += 4) {
+          const auto p = v[i].x, q = v[i].y;
+          v[i].x = p + q;
+          v[i].y = p - q;
+          __stcg(row + 32 * i, v[i]);
+        }
+      }
+    } else {
+      wait_prior_grid();  // the previous stage's rows
+      const uint32_t unit = sub * G + w;  // block of 2^(11-HI) columns
+      const T *col = inter + ((size_t)unit << (11 - HI));
+      double s[NQ + 1];
+      if constexpr (HI <= 5) {
+        // register i: row i mod 2^HI, column block i >> HI of 64 columns (a pair per lane)
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+          v[i] = __ldcg(reinterpret_cast<const V *>(col + (size_t)(i & (NROW - 1)) * ROW + 64 * (i >> HI)) + lane);
+      } else {
+        // lane: column in its low 11 - HI bits, the row's low HI - 6 bits above them;
+        // register pair i: rows with bits HI-6 = (x, y) and i above
+        constexpr int CB = 11 - HI, LB = HI - 6;
+        const T *p = col + (lane & ((1 << CB) - 1)) + (size_t)(lane >> CB) * ROW;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          v[i].x = __ldcg(p + (size_t)((2 * i) << LB) * ROW);
+          v[i].y = __ldcg(p + (size_t)((2 * i + 1) << LB) * ROW);
+        }
+#pragma unroll
+        for (int m = 1 << CB; m < 32; m <<= 1) lane_wht(v, lane, m);
+      }
+      if constexpr (QS == QS_GEN) group_sync<32 * G>(1 + grp);  // the moments stage in the buffer
+      wide_moments<QS, (HI <= 5 ? HI : 5), (HI > 5)>(v, s, a.qp, buf + 2048 * w, lane);
+      // The columns are dead once read (their slot is rewritten two stages later, after
+      // griddepcontrol.wait on the launch in between): drop their L2 lines without writing
+      // them back.  A unit owns whole 128-byte lines when its row chunk is at least that.
+      constexpr uint32_t CHUNK = (2048u >> HI) * sizeof(T);
+      if constexpr (CHUNK >= 128) {
+        constexpr uint32_t LPR = CHUNK / 128;  // lines per row
+        __syncwarp();                          // every lane's reads come before
+#pragma unroll
+        for (uint32_t ln = lane; ln < NROW * LPR; ln += 32)
+          asm volatile("discard.global.L2 [%0], 128;" ::"l"(reinterpret_cast<const char *>(
+                           col + (size_t)(ln / LPR) * ROW) + (ln % LPR) * 128)
+                       : "memory");
+      }
+      s[0] = x == 0 ? s[0] : 4.0 * s[0];
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) s[1 + q] *= q_scale<QS>(q, x == 0, a.qp);
+#pragma unroll
+      for (int q = 0; q <= NQ; ++q) dd_add(acc[q], s[q]);
+    }
+  }
+  if (n2 > 0) {
+    // fixed-order butterfly reduction of the lanes' accumulators
+#pragma unroll
+    for (int q = 0; q <= NQ; ++q) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        dd other;
+        other.hi = __shfl_xor_sync(0xffffffffu, acc[q].hi, o);
+        other.lo = __shfl_xor_sync(0xffffffffu, acc[q].lo, o);
+        dd_add_dd(acc[q], other);
+      }
+    }
+    if (lane == 0) {
+      wait_prior_grid();  // the previous stage updates the same slot
+      double *sl = a.slots + ((size_t)blockIdx.x * WideCta<G>::WARPS + warp) * 2 * (NQ + 1);
+#pragma unroll
+      for (int q = 0; q <= NQ; ++q) {
+        dd d{sl[2 * q], sl[2 * q + 1]};
+        dd_add_dd(d, acc[q]);
+        sl[2 * q] = d.hi;
+        sl[2 * q + 1] = d.lo;
+      }
+    }
+  }
 }
 
 }  // namespace hm

@@ -31,3 +31,28 @@ def test_single_cta_ranges(ctx, hm, n, qs, precision):
             N.set_param(N.HM_PARAM_ENGINE, 0)
         assert p2.sum() == pytest.approx(p2r.sum(), rel=tol)
         assert m.sum(axis=1) == pytest.approx(mr.sum(axis=1), rel=tol)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("qs", sorted(QS))
+@pytest.mark.parametrize("n", [15, 16, 17, 18, 19, 20, 21])
+def test_two_pass_ranges(ctx, hm, n, qs, precision):
+    N = hm._native
+    psi = rand_state(1 << n, 900 + n)
+    full = 1 << n
+    tol = 1e-13 if precision == "fp64" else 1e-6
+    ranges = [(0, 1), (0, 5), (1021, 1034)] if n >= 19 else [(0, 1), (0, 150), (1, 2), (3000, 3333), (full - 37, full)]
+    for kb, ke in ranges:
+        p2, m = ctx.sre_range(psi, kb, ke, QS[qs], hm.PRECISIONS[precision])
+        try:
+            N.set_param(N.HM_PARAM_BATCH, 3)  # several stages, the last one not full
+            p2s, ms = ctx.sre_range(psi, kb, ke, QS[qs], hm.PRECISIONS[precision])
+            N.set_param(N.HM_PARAM_BATCH, 0)
+            N.set_param(N.HM_PARAM_ENGINE, 2)
+            p2r, mr = ctx.sre_range(psi, kb, ke, QS[qs], hm.PRECISIONS[precision])
+        finally:
+            N.set_param(N.HM_PARAM_BATCH, 0)
+            N.set_param(N.HM_PARAM_ENGINE, 0)
+        for p, v in ((p2, m), (p2s, ms)):
+            assert p.sum() == pytest.approx(p2r.sum(), rel=tol)
+            assert v.sum(axis=1) == pytest.approx(mr.sum(axis=1), rel=tol)
