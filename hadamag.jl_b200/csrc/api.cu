@@ -161,7 +161,7 @@ int hm_destroy(hm_ctx *c) {
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
   void *dev[] = {c->d_psi, c->d_psi32, c->d_inter, c->d_partials, c->d_ctrl, c->d_out, c->d_aux, c->d_aux2,
-                 c->d_queue};
+                 c->d_queue, c->d_ticket};
   for (void *p : dev)
     if (p) cudaFree(p);
   if (c->h_out) cudaFreeHost(c->h_out);
@@ -321,51 +321,37 @@ int hm_sre_batched(hm_ctx *c, int nstates, const double *const *psis, const int 
                                c->stream));
     off += len;
   }
-  // states below the split size go through one persistent queue launch (FP32: plus one
-  // FP64 launch of every state's x = 0 transform); from the split size up a state's own
-  // sweep dwarfs a call's fixed cost and the stage kernels are faster per X-string than
-  // the queue (no dead-tile write-back), so those states, n > 21 and the plain selector
-  // run one state per call
+  // states below the split size (one-warp transforms) go through one persistent queue launch
+  // (FP32: plus one FP64 launch of their x = 0 transforms); from the split size up a sweep
+  // fills the GPU by itself and its own kernels are faster than the queue's units (one CTA
+  // per X-string for n = 12 .. 14 half their time, no dead-tile write-back above), so those
+  // states are swept one after the other and read back together
   c->launches = 0;
   const int split_n = hm::queue_cfg().batch_split_n;
-  auto queued = [&](int n) { return precision != HM_PLAIN && n < split_n && n <= 21; };
-  std::vector<QueueItem> items;
-  std::vector<int> where;
+  std::vector<QueueItem> items[2];
+  std::vector<int> where[2];
   off = 0;
   for (int s = 0; s < nstates; ++s) {
     const size_t len = (size_t)1 << ns[s];
-    if (queued(ns[s])) {
-      items.push_back(QueueItem{(const double2 *)c->d_psi + off, ns[s], 0, (uint64_t)len});
-      where.push_back(s);
-    }
+    const int own = precision != HM_PLAIN && ns[s] < split_n && ns[s] <= 21 ? 0 : 1;
+    items[own].push_back(QueueItem{(const double2 *)c->d_psi + off, ns[s], 0, (uint64_t)len});
+    where[own].push_back(s);
     off += len;
   }
-  std::vector<double> dd((size_t)nstates * 2 * (1 + nq));
+  const int w = 2 * (1 + nq);
+  std::vector<double> dd((size_t)nstates * w);
   double total_ms = 0.0;
-  long long launches = 0;
-  if (!items.empty()) {
-    std::vector<double> qdd(items.size() * 2 * (1 + nq));
-    HM_TRY(run_queue_sre(c, items.data(), (int)items.size(), q, precision, qdd.data()));
+  for (int own = 0; own < 2; ++own) {
+    if (items[own].empty()) continue;
+    std::vector<double> part(items[own].size() * w);
+    HM_TRY(own ? run_sre_states(c, items[own].data(), (int)items[own].size(), q, precision, part.data())
+               : run_queue_sre(c, items[own].data(), (int)items[own].size(), q, precision, part.data()));
     total_ms += c->last_ms;
-    launches += c->launches;
-    for (size_t i = 0; i < items.size(); ++i)
-      std::copy(qdd.begin() + i * 2 * (1 + nq), qdd.begin() + (i + 1) * 2 * (1 + nq),
-                dd.begin() + (size_t)where[i] * 2 * (1 + nq));
-  }
-  off = 0;
-  for (int s = 0; s < nstates; ++s) {
-    const size_t len = (size_t)1 << ns[s];
-    if (!queued(ns[s])) {
-      c->launches = 0;
-      HM_TRY(run_sre(c, (const double2 *)c->d_psi + off, ns[s], 0, len, q, precision, dd.data() + (size_t)s * 2 * (1 + nq)));
-      total_ms += c->last_ms;
-      launches += c->launches;
-    }
-    off += len;
+    for (size_t i = 0; i < items[own].size(); ++i)
+      std::copy(part.begin() + i * w, part.begin() + (i + 1) * w, dd.begin() + (size_t)where[own][i] * w);
   }
   for (int s = 0; s < nstates; ++s) sre_finish(dd.data() + (size_t)s * 2 * (1 + nq), ns[s], nq, out_sre + (size_t)s * nq, out_lost + s);
   c->last_ms = total_ms;
-  c->launches = launches;
   return HM_OK;
 }
 

@@ -7,6 +7,7 @@
 #include <string.h>
 
 #include <string>
+#include <unordered_map>
 
 #include "../../include/hadamag_b200.h"
 
@@ -41,6 +42,8 @@ struct hm_ctx {
   size_t h_out_cap = 0;
   void *h_pin = nullptr;  // pinned host scratch
   size_t h_pin_cap = 0;
+  unsigned *d_ticket = nullptr;  // CTAs of the current launch that are done (see fold_last)
+  std::unordered_map<const void *, int> occ;  // CTAs per SM of the kernels launched so far
   void *d_queue = nullptr;  // queue sweep: state table, batch counters, per-warp slots
   size_t queue_cap = 0;
 };
@@ -116,6 +119,23 @@ inline int ensure_host(hm_ctx *c, void **p, size_t *cap, size_t bytes) {
   return HM_OK;
 }
 
+// Dynamic shared memory limit and CTAs per SM of a kernel, asked for once per context (the
+// two queries cost a small call 3 us each time).
+template <typename Kern>
+inline int kernel_occ(hm_ctx *c, Kern kern, int threads, size_t smem, int *occ) {
+  const void *key = reinterpret_cast<const void *>(kern);
+  const auto it = c->occ.find(key);
+  if (it != c->occ.end()) {
+    *occ = it->second;
+    return HM_OK;
+  }
+  HM_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int n = 0;
+  HM_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem));
+  c->occ[key] = *occ = n < 1 ? 1 : n;
+  return HM_OK;
+}
+
 struct QReq {
   double q[4];
   int nq;
@@ -141,7 +161,7 @@ struct QueueCfg {
   int engine = 0;  // single-state sweeps: 0 automatic, 1 stage kernels, 2 queue sweep
   int stall_test = 0;  // test of the bounded waits (HM_PARAM_QUEUE_STALL_TEST)
   int lead = 2;        // batches between a batch's pass 1 and pass 2 (HM_PARAM_QUEUE_LEAD)
-  int batch_split_n = 15;  // hm_sre_batched: states from this n up run one per call (HM_PARAM_BATCH_SPLIT_N)
+  int batch_split_n = 12;  // hm_sre_batched: states from this n up have a sweep each (HM_PARAM_BATCH_SPLIT_N)
   int tuned_x[2][32] = {};
   int tuned_cps[2][32] = {};
   int tuned_engine[2][32] = {};  // hm_autotune's choice per (precision, n): 0 none, 1 stage, 2 queue
@@ -159,6 +179,9 @@ int run_queue_sre(hm_ctx *c, const QueueItem *items, int nitems, const QReq &q, 
 // out_dd (host): [p2_hi, p2_lo, m0_hi, m0_lo, ...] for each requested q.
 int run_sre(hm_ctx *c, const double2 *psi_dev, int n, uint64_t kb, uint64_t ke, const QReq &q, int precision,
             double *out_dd);
+// exact SRE raw sums of several states, one sweep after the other, read back together;
+// out_dd per item as run_queue
+int run_sre_states(hm_ctx *c, const QueueItem *items, int nitems, const QReq &q, int precision, double *out_dd);
 int run_sre_plain(hm_ctx *c, const double2 *psi_dev, int n, uint64_t kb, uint64_t ke, const QReq &q,
                   double *out_dd);
 

@@ -3,5 +3,6 @@
 #include "sre_launch.cuh"
 
 namespace hm {
-template int launch_sre_qs<float, 32, QS_Q2>(hm_ctx *, const void *, int, uint64_t, uint64_t, const QParams &, int *);
+template int launch_sre_qs<float, 32, QS_Q2>(hm_ctx *, const void *, int, uint64_t, uint64_t, const QParams &, double *,
+                                                int *);
 }

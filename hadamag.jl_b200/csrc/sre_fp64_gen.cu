@@ -3,5 +3,6 @@
 #include "sre_launch.cuh"
 
 namespace hm {
-template int launch_sre_qs<double, 32, QS_GEN>(hm_ctx *, const void *, int, uint64_t, uint64_t, const QParams &, int *);
+template int launch_sre_qs<double, 32, QS_GEN>(hm_ctx *, const void *, int, uint64_t, uint64_t, const QParams &, double *,
+                                                int *);
 }

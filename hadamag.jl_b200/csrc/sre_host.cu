@@ -10,19 +10,16 @@
 
 namespace hm {
 
-template <typename T, int R, int QS>
-int launch_sre_qs(hm_ctx *c, const void *psi_dev, int n, uint64_t kb, uint64_t ke, const QParams &qp, int *nwarps);
-
 template <typename T>
 static int launch_sre_prec(hm_ctx *c, const void *psi_dev, int n, uint64_t kb, uint64_t ke, int kind,
-                           const QParams &qp, int *nwarps) {
+                           const QParams &qp, double *out, int *nwarps) {
   switch (kind) {
     case QS_Q2:
-      return launch_sre_qs<T, 32, QS_Q2>(c, psi_dev, n, kb, ke, qp, nwarps);
+      return launch_sre_qs<T, 32, QS_Q2>(c, psi_dev, n, kb, ke, qp, out, nwarps);
     case QS_Q23:
-      return launch_sre_qs<T, 32, QS_Q23>(c, psi_dev, n, kb, ke, qp, nwarps);
+      return launch_sre_qs<T, 32, QS_Q23>(c, psi_dev, n, kb, ke, qp, out, nwarps);
     default:
-      return launch_sre_qs<T, 32, QS_GEN>(c, psi_dev, n, kb, ke, qp, nwarps);
+      return launch_sre_qs<T, 32, QS_GEN>(c, psi_dev, n, kb, ke, qp, out, nwarps);
   }
 }
 
@@ -179,23 +176,12 @@ int run_queue_sre(hm_ctx *c, const QueueItem *items, int nitems, const QReq &q, 
   return HM_OK;
 }
 
-int run_sre(hm_ctx *c, const double2 *psi_dev, int n, uint64_t kb, uint64_t ke, const QReq &q, int precision,
-            double *out_dd) {
-  if (precision == HM_PLAIN || n > 24 || n < 1) return run_sre_plain(c, psi_dev, n, kb, ke, q, out_dd);
-  if (ke <= kb) {
-    for (int i = 0; i < 2 * (1 + q.nq); ++i) out_dd[i] = 0.0;
-    return HM_OK;
-  }
-  if (n >= 12 && n <= 21 && sweep_engine(n, precision) == 2) {
-    const QueueItem it{psi_dev, n, kb, ke};
-    return run_queue_sre(c, &it, 1, q, precision, out_dd);
-  }
-  QParams qp;
-  int idx[4];
-  const int kind = choose_qs(q, qp, idx);
-  const int nsum = 1 + (kind == QS_Q2 ? 1 : (kind == QS_Q23 ? 2 : 4));
+// Launches the sweep of [kb, ke) and leaves its raw sums (2 nsum doubles) in `out`, page-locked
+// host memory, once the stream gets there.  FP32 callers keep x = 0 out of the range.
+static int enqueue_sweep(hm_ctx *c, const double2 *psi_dev, int n, uint64_t kb, uint64_t ke, int kind,
+                         const QParams &qp, int nsum, int precision, double *out) {
   const uint64_t len = 1ull << n;
-  // the fused kernels (n <= 11) read the FP64 state in both precisions; the FP32 two-pass
+  // the fused kernels (n <= 11) read the FP64 state in both precisions; the larger FP32
   // kernels read an FP32 copy
   const void *psi_k = psi_dev;
   if (precision == HM_FP32 && (n - 1) > 10) {
@@ -205,49 +191,87 @@ int run_sre(hm_ctx *c, const double2 *psi_dev, int n, uint64_t kb, uint64_t ke, 
     HM_CUDA(c, cudaGetLastError());
     psi_k = c->d_psi32;
   }
-  // x = 0 (F = WHT of |psi|^2, whose F(0)^4 = 1 can dominate m) always runs in FP64: the
-  // FP64 kernels build it themselves (top-bit pairing in pass 1, scale 1), and an FP32 call
-  // runs it as an FP64 call of its own, since the FP32 kernels would round it
-  const bool split_zero = kb == 0 && precision == HM_FP32;
-  const uint64_t kb_main = split_zero ? 1 : kb;
   int nwarps = 0;
-  HM_CUDA(c, cudaEventRecord(c->ev0, c->stream));
-  if (kb_main >= ke) {
-    // only x = 0 requested: the main kernels have nothing to do
-    HM_TRY(ensure_dev(c, (void **)&c->d_partials, &c->partials_cap, sizeof(double) * 16));
-    HM_CUDA(c, cudaMemsetAsync(c->d_partials, 0, sizeof(double) * 2 * nsum, c->stream));
-    nwarps = 1;
-  } else if (precision == HM_FP32) {
-    HM_TRY((launch_sre_prec<float>(c, psi_k, n, kb_main, ke, kind, qp, &nwarps)));
+  if (precision == HM_FP32) {
+    HM_TRY((launch_sre_prec<float>(c, psi_k, n, kb, ke, kind, qp, out, &nwarps)));
   } else {
-    HM_TRY((launch_sre_prec<double>(c, psi_k, n, kb_main, ke, kind, qp, &nwarps)));
+    HM_TRY((launch_sre_prec<double>(c, psi_k, n, kb, ke, kind, qp, out, &nwarps)));
+  }
+  if (nwarps > 0) {
+    k_fold_partials<<<1, 256, 0, c->stream>>>(c->d_partials, nwarps, nsum, out);
+    c->launches += 1;
+    HM_CUDA(c, cudaGetLastError());
+  }
+  return HM_OK;
+}
+
+// Sweeps of several states one after the other, read back together: every sweep writes its
+// sums to its own page-locked slot, and the host waits once.  FP32: x = 0 (F = WHT of
+// |psi|^2, whose F(0)^4 = 1 can dominate m) is an FP64 sweep of its own, since the FP32
+// kernels would round it; the FP64 kernels build it themselves.
+static int run_sweeps(hm_ctx *c, const QueueItem *items, int nitems, const QReq &q, int precision, double *out_dd) {
+  constexpr int SLOT = 16;
+  QParams qp;
+  int idx[4];
+  const int kind = choose_qs(q, qp, idx);
+  const int nsum = 1 + (kind == QS_Q2 ? 1 : (kind == QS_Q23 ? 2 : 4)), w = 2 * (1 + q.nq);
+  HM_TRY(ensure_host(c, (void **)&c->h_out, &c->h_out_cap, sizeof(double) * 2 * SLOT * (size_t)nitems + 64));
+  if (!c->d_ticket) {
+    HM_CUDA(c, cudaMalloc((void **)&c->d_ticket, 256));
+    HM_CUDA(c, cudaMemsetAsync(c->d_ticket, 0, 256, c->stream));
+  }
+  HM_CUDA(c, cudaEventRecord(c->ev0, c->stream));
+  for (int i = 0; i < nitems; ++i) {
+    const QueueItem &it = items[i];
+    double *slot = c->h_out + (size_t)2 * SLOT * i;
+    memset(slot, 0, sizeof(double) * 2 * SLOT);
+    const bool zero = precision == HM_FP32 && it.kb == 0 && it.ke > 0;
+    const uint64_t kb = it.kb + (zero ? 1 : 0);
+    if (kb < it.ke) HM_TRY(enqueue_sweep(c, it.psi, it.n, kb, it.ke, kind, qp, nsum, precision, slot));
+    if (zero) HM_TRY(enqueue_sweep(c, it.psi, it.n, 0, 1, kind, qp, nsum, HM_FP64, slot + SLOT));
   }
   HM_CUDA(c, cudaEventRecord(c->ev1, c->stream));
-  HM_TRY(ensure_dev(c, (void **)&c->d_out, &c->out_cap, sizeof(double) * 16));
-  k_fold_partials<<<1, 256, 0, c->stream>>>(c->d_partials, nwarps, nsum, c->d_out);
-  c->launches += 1;
-  HM_CUDA(c, cudaGetLastError());
-  HM_TRY(ensure_host(c, (void **)&c->h_out, &c->h_out_cap, sizeof(double) * 16 + 64));
-  HM_CUDA(c, cudaMemcpyAsync(c->h_out, c->d_out, sizeof(double) * 2 * nsum, cudaMemcpyDeviceToHost, c->stream));
   HM_CUDA(c, cudaStreamSynchronize(c->stream));
   float ms = 0.f;
   HM_CUDA(c, cudaEventElapsedTime(&ms, c->ev0, c->ev1));
   c->last_ms = ms;
-  out_dd[0] = c->h_out[0];
-  out_dd[1] = c->h_out[1];
-  for (int i = 0; i < q.nq; ++i) {
-    out_dd[2 + 2 * i] = c->h_out[2 * idx[i]];
-    out_dd[3 + 2 * i] = c->h_out[2 * idx[i] + 1];
+  for (int i = 0; i < nitems; ++i) {
+    const double *slot = c->h_out + (size_t)2 * SLOT * i;
+    double *o = out_dd + (size_t)w * i;
+    for (int t = 0; t <= q.nq; ++t) {
+      const int at = t == 0 ? 0 : 2 * idx[t - 1];
+      o[2 * t] = slot[at];
+      o[2 * t + 1] = slot[at + 1];
+      dd_add_host(o + 2 * t, slot[SLOT + at], slot[SLOT + at + 1]);
+    }
   }
-  if (split_zero) {
-    // x = 0 (F = WHT of |psi|^2) is not part of the stage kernels' sweep: one FP64
-    // transform of the queue sweep, added as a double-double term
-    const double ms_main = c->last_ms;
-    double z[10];
-    HM_TRY(run_sre(c, psi_dev, n, 0, 1, q, HM_FP64, z));
-    c->last_ms += ms_main;
-    for (int t = 0; t < 1 + q.nq; ++t) dd_add_host(out_dd + 2 * t, z[2 * t], z[2 * t + 1]);
+  return HM_OK;
+}
+
+int run_sre(hm_ctx *c, const double2 *psi_dev, int n, uint64_t kb, uint64_t ke, const QReq &q, int precision,
+            double *out_dd) {
+  if (precision == HM_PLAIN || n > 24 || n < 1) return run_sre_plain(c, psi_dev, n, kb, ke, q, out_dd);
+  if (ke <= kb) {
+    for (int i = 0; i < 2 * (1 + q.nq); ++i) out_dd[i] = 0.0;
+    return HM_OK;
   }
+  const QueueItem it{psi_dev, n, kb, ke};
+  if (n >= 12 && n <= 21 && sweep_engine(n, precision) == 2) return run_queue_sre(c, &it, 1, q, precision, out_dd);
+  return run_sweeps(c, &it, 1, q, precision, out_dd);
+}
+
+int run_sre_states(hm_ctx *c, const QueueItem *items, int nitems, const QReq &q, int precision, double *out_dd) {
+  bool one_wait = precision != HM_PLAIN;
+  for (int i = 0; i < nitems; ++i)
+    if (items[i].n >= 12 && items[i].n <= 21 && sweep_engine(items[i].n, precision) == 2) one_wait = false;
+  if (one_wait) return nitems > 0 ? run_sweeps(c, items, nitems, q, precision, out_dd) : HM_OK;
+  double ms = 0.0;
+  for (int i = 0; i < nitems; ++i) {
+    HM_TRY(run_sre(c, items[i].psi, items[i].n, items[i].kb, items[i].ke, q, precision,
+                   out_dd + (size_t)2 * (1 + q.nq) * i));
+    ms += c->last_ms;
+  }
+  c->last_ms = ms;
   return HM_OK;
 }
 

@@ -74,10 +74,8 @@ static int launch_fused(hm_ctx *c, const SreArgs &a0, int *nwarps_out) {
   constexpr int PB = ilog2c(R) + 5;
   const size_t smem = (size_t)FUSED_WARPS * 32 * R * sizeof(V);
   auto kern = k_sre_fused<T, R, NB, QS>;
-  HM_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int occ = 0;
-  HM_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, FUSED_WARPS * 32, smem));
-  if (occ < 1) occ = 1;
+  HM_TRY(kernel_occ(c, kern, FUSED_WARPS * 32, smem, &occ));
   const uint64_t XPW = 1ull << (PB - NB);
   const uint64_t ngroups = (a.k_end - a.k_begin + XPW - 1) / XPW;
   uint64_t blocks = (ngroups + FUSED_WARPS - 1) / FUSED_WARPS;
@@ -91,7 +89,7 @@ static int launch_fused(hm_ctx *c, const SreArgs &a0, int *nwarps_out) {
   kern<<<(unsigned)blocks, FUSED_WARPS * 32, smem, c->stream>>>(a);
   c->launches += 1;
   HM_CUDA(c, cudaGetLastError());
-  *nwarps_out = nwarps;
+  *nwarps_out = 0;  // folded by the kernel
   return HM_OK;
 }
 
@@ -103,10 +101,8 @@ static int launch_wide(hm_ctx *c, const SreArgs &a0, int *nwarps_out) {
   SreArgs a = a0;
   const size_t smem = (size_t)2048 * G * sizeof(T);
   auto kern = k_sre_wide<T, G, QS>;
-  HM_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int occ = 0;
-  HM_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 32 * G, smem));
-  if (occ < 1) occ = 1;
+  HM_TRY(kernel_occ(c, kern, 32 * G, smem, &occ));
   const uint64_t blocks = std::min<uint64_t>(a.k_end - a.k_begin, (uint64_t)c->num_sms * occ);
   const int nwarps = (int)blocks * G;
   HM_TRY(ensure_dev(c, (void **)&c->d_partials, &c->partials_cap,
@@ -115,7 +111,7 @@ static int launch_wide(hm_ctx *c, const SreArgs &a0, int *nwarps_out) {
   kern<<<(unsigned)blocks, 32 * G, smem, c->stream>>>(a);
   c->launches += 1;
   HM_CUDA(c, cudaGetLastError());
-  *nwarps_out = nwarps;
+  *nwarps_out = 0;  // folded by the kernel
   return HM_OK;
 }
 
@@ -231,10 +227,8 @@ static int launch_stages(hm_ctx *c, const SreArgs &a0, int *nwarps_out) {
   }
   const size_t smem = (size_t)SRE_WARPS * 32 * R * sizeof(V);
   auto kern = k_sre_stage<T, R, HI, QS>;
-  HM_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int occ = 0;
-  HM_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, SRE_WARPS * 32, smem));
-  if (occ < 1) occ = 1;
+  HM_TRY(kernel_occ(c, kern, SRE_WARPS * 32, smem, &occ));
   long long units = 2 * (long long)X * (long long)U;
   int blocks = c->num_sms * occ;
   if ((long long)blocks * SRE_WARPS > units) blocks = (int)((units + SRE_WARPS - 1) / SRE_WARPS);
@@ -293,10 +287,8 @@ static int launch_wide_stages(hm_ctx *c, const SreArgs &a0, int *nwarps_out) {
   a.ring = c->d_inter;
   const size_t smem = (size_t)WARPS * 2048 * sizeof(T);
   auto kern = k_sre_wide_stage<T, G, HI, QS>;
-  HM_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int occ = 0;
-  HM_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, WARPS * 32, smem));
-  if (occ < 1) occ = 1;
+  HM_TRY(kernel_occ(c, kern, WARPS * 32, smem, &occ));
   const long long items = 2 * (long long)X << HI;
   const int blocks = (int)std::min<long long>((long long)c->num_sms * occ, (items * G + WARPS - 1) / WARPS);
   const int nwarps = blocks * WARPS;
@@ -355,10 +347,8 @@ static int launch_stages3(hm_ctx *c, const SreArgs &a0, int *nwarps_out) {
   }
   const size_t smem = (size_t)SRE_WARPS * 32 * R * sizeof(V);
   auto kern = k_sre_stage3<T, R, K, QS>;
-  HM_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int occ = 0;
-  HM_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, SRE_WARPS * 32, smem));
-  if (occ < 1) occ = 1;
+  HM_TRY(kernel_occ(c, kern, SRE_WARPS * 32, smem, &occ));
   const long long units = (long long)X * (long long)U;
   int blocks = c->num_sms * occ;
   if ((long long)blocks * SRE_WARPS > units) blocks = (int)((units + SRE_WARPS - 1) / SRE_WARPS);
@@ -408,7 +398,10 @@ static int dispatch_sre(hm_ctx *c, const SreArgs &a, int *nw) {
       case 3:
         return launch_wide<T, 8, QS>(c, a, nw);
       case 4:
-        return launch_wide_stages<T, 15, QS>(c, a, nw);
+        if constexpr (sizeof(T) == 4)
+          return launch_wide<T, 16, QS>(c, a, nw);
+        else
+          return launch_wide_stages<T, 15, QS>(c, a, nw);
       case 5:
         return launch_wide_stages<T, 16, QS>(c, a, nw);
       case 6:
@@ -443,12 +436,15 @@ static int dispatch_sre(hm_ctx *c, const SreArgs &a, int *nw) {
   return set_err(c, HM_ERR_SIZE, "n = %d outside the fused range of this precision", a.n);
 }
 
-// one precision and moment set; returns the number of per-warp partial records written
+// One precision and moment set.  nwarps = 0: the kernel wrote the folded sums to `out`;
+// otherwise the number of per-warp partial records left to fold.
 template <typename T, int R, int QS>
 int launch_sre_qs(hm_ctx *c, const void *psi_dev, int n, uint64_t kb, uint64_t ke, const QParams &qp,
-                  int *nwarps) {
+                  double *out, int *nwarps) {
   SreArgs a;
   memset(&a, 0, sizeof a);
+  a.out = out;
+  a.ticket = c->d_ticket;
   a.psi = psi_dev;
   a.n = n;
   a.k_begin = kb;
@@ -460,7 +456,7 @@ int launch_sre_qs(hm_ctx *c, const void *psi_dev, int n, uint64_t kb, uint64_t k
 // one translation unit per precision and moment set holds the kernels (sre_fp64_q2.cu, ...)
 #define HM_EXTERN_SRE(T, QS)                                                                             \
   extern template int launch_sre_qs<T, 32, QS>(hm_ctx *, const void *, int, uint64_t, uint64_t,          \
-                                               const QParams &, int *);
+                                               const QParams &, double *, int *);
 HM_EXTERN_SRE(double, QS_Q2)
 HM_EXTERN_SRE(double, QS_Q23)
 HM_EXTERN_SRE(double, QS_GEN)

@@ -1,6 +1,6 @@
-// sre_wide.cuh -- exact-SRE transforms held by a group of G warps (G = 2, 4, 8): the whole
-// transform of an X-string for n = 12, 13, 14 (2^(n-1) = 1024 G complex values) without
-// leaving the SM.
+// sre_wide.cuh -- exact-SRE transforms held by a group of G warps (G = 2, 4, 8, in FP32 also
+// 16): the whole transform of an X-string for n = 12, 13, 14 (FP32 also 15; 2^(n-1) = 1024 G
+// complex values) without leaving the SM, and the two-pass sweep of larger n.
 //
 // The WHT is real-linear, so the real and imaginary parts separate after the products:
 //   phase A  lane l, register i of warp w holds the complex element e = 32 i + l + 1024 w:
@@ -17,6 +17,7 @@
 // the kernel, two-pass stages -> this (us):
 //   q = 2   FP64  n = 12: 69 -> 31   n = 13: 226 -> 124   n = 14: 1107 -> 530
 //           FP32  n = 12: 60 -> 32   n = 13: 144 -> 81    n = 14: 614 -> 308
+//                 n = 15: 2180 -> 1430 (2030 with the two-pass sweep below)
 //   n = 13, FP64: q = 2 and 3 231 -> 137, q = 4 724 -> 291, q = 2.5 1498 -> 1032
 // FP64 at n = 13 is 1.04 clocks per complex element and SM, 0.55 of them FP64 issue.
 #pragma once
@@ -65,12 +66,14 @@ __device__ __forceinline__ void group_sync(int id) {
 }
 
 // position of real element e of a plane in the group's buffer: 16-byte granules XOR-ed with
-// bits 5 .. 7 of e, so that both the phase-A stores (lanes over bits 0 .. 4) and the phase-B
-// loads (lanes over bits 5 .. 9, 16 bytes each) are free of bank conflicts
-template <typename T>
+// bits 5 .. 7 of e (G = 16: bits 5, 6 and 11), the low three bits of the phase-B lane, so
+// that both the phase-A stores (lanes over bits 0 .. 4) and the phase-B loads (16 bytes a
+// lane) are free of bank conflicts
+template <typename T, int G>
 __device__ __forceinline__ uint32_t wide_pos(uint32_t e) {
   constexpr int GS = sizeof(T) == 8 ? 1 : 2;  // log2 of the values per granule
-  return e ^ (((e >> 5) & 7u) << GS);
+  const uint32_t f = G == 16 ? ((e >> 5) & 3u) | ((e >> 9) & 4u) : (e >> 5) & 7u;
+  return e ^ (f << GS);
 }
 
 // phase A's 32 complex registers -> the two planes
@@ -81,7 +84,7 @@ __device__ __forceinline__ void wide_put(V (&v)[32], T *buf, int w, int lane) {
     wht_class<2, 5>(v, c);
 #pragma unroll
     for (int i = c; i < 32; i += 4) {
-      const uint32_t p = wide_pos<T>((uint32_t)(32 * i + lane)) + 1024u * w;
+      const uint32_t p = wide_pos<T, G>((uint32_t)(32 * i + lane) + 1024u * w);
       buf[p] = v[i].x;
       buf[1024 * G + p] = v[i].y;
     }
@@ -93,14 +96,17 @@ __device__ __forceinline__ void wide_put(V (&v)[32], T *buf, int w, int lane) {
 //   G = 2: lanes 5 6 7 8 9,     warp: plane
 //   G = 4: lanes 5 6 7 8 11,    warp: 9, plane
 //   G = 8: lanes 5 6 7 11 12,   warp: 8, 9, plane
+//   G = 16: lanes 5 6 11 12 13, warp: 7, 8, 9, plane
 template <int G>
 __device__ __forceinline__ uint32_t wide_base(int w, int lane) {
   if constexpr (G == 2) {
     return (uint32_t)lane << 5;
   } else if constexpr (G == 4) {
     return ((uint32_t)(lane & 15) << 5) | ((uint32_t)(lane >> 4) << 11) | ((uint32_t)(w & 1) << 9);
-  } else {
+  } else if constexpr (G == 8) {
     return ((uint32_t)(lane & 7) << 5) | ((uint32_t)(lane >> 3) << 11) | ((uint32_t)(w & 3) << 8);
+  } else {
+    return ((uint32_t)(lane & 3) << 5) | ((uint32_t)(lane >> 2) << 11) | ((uint32_t)(w & 7) << 7);
   }
 }
 
@@ -115,11 +121,11 @@ __device__ __forceinline__ void wide_get(V (&v)[32], const T *buf, int w, int la
     if constexpr (sizeof(T) == 8) {
 #pragma unroll
       for (int i = 0; i < 16; ++i)
-        v[16 * b + i] = *reinterpret_cast<const V *>(plane + wide_pos<T>((base | (2 * i))) + 1024 * b);
+        v[16 * b + i] = *reinterpret_cast<const V *>(plane + wide_pos<T, G>(base | (2 * i)) + 1024 * b);
     } else {
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const float4 q = *reinterpret_cast<const float4 *>(plane + wide_pos<T>((base | (4 * i))) + 1024 * b);
+        const float4 q = *reinterpret_cast<const float4 *>(plane + wide_pos<T, G>(base | (4 * i)) + 1024 * b);
         v[16 * b + 2 * i] = make_float2(q.x, q.y);
         v[16 * b + 2 * i + 1] = make_float2(q.z, q.w);
       }
@@ -294,6 +300,11 @@ __device__ __forceinline__ void wide_lane_bits(V (&v)[32], int lane) {
     lane_wht(v, lane, 8);
     lane_wht(v, lane, 16);
   }
+  if constexpr (G == 16) {
+    lane_wht(v, lane, 4);
+    lane_wht(v, lane, 8);
+    lane_wht(v, lane, 16);
+  }
 }
 
 // Groups per SM: FP64 8 warps (255 registers), FP32 16 warps (128 registers).
@@ -342,6 +353,7 @@ __global__ void __launch_bounds__(32 * G, WideOcc<T, G>::value) k_sre_wide(SreAr
     }
   }
   if (lane == 0) write_partials<NQ>(a.partials, blockIdx.x * G + w, acc);
+  fold_last<NQ, 32 * G>(a, (int)gridDim.x * G);
 }
 
 // ---------------------------------------------------------------------------------

@@ -102,7 +102,7 @@ int hm_set_stream(hm_ctx *ctx, void *cuda_stream);
  * (1..16, default 2; the ring keeps at least lead + 1 slots). */
 #define HM_PARAM_QUEUE_LEAD 12
 /* HM_PARAM_BATCH_SPLIT_N: hm_sre_batched runs states with n below this (1..22, default
- * 15) in one queue launch and the others one state per call (22: every state up to n = 21
+ * 12) in one queue launch and the others with a sweep each (22: every state up to n = 21
  * in the queue). */
 #define HM_PARAM_BATCH_SPLIT_N 14
 int hm_set_param(int param, int value);
@@ -194,8 +194,8 @@ int hm_multi_release(void);
 
 /* Batched exact SRE of many states of possibly different qubit counts (no reference
  * counterpart; the reference handles one state per call): one upload of every state, one
- * persistent queue launch for the states below HM_PARAM_BATCH_SPLIT_N, one call's kernels
- * per larger state.  psis[s] points to 2^ns[s] interleaved complex doubles (host).  For
+ * persistent queue launch for the states below HM_PARAM_BATCH_SPLIT_N, one sweep per larger
+ * state, all read back together.  psis[s] points to 2^ns[s] interleaved complex doubles (host).  For
  * each state s and each q: out_sre[s*nq + i]; out_lost[s]. */
 int hm_sre_batched(hm_ctx *ctx, int nstates, const double *const *psis, const int *ns, const double *qs, int nq,
                    int precision, double *out_sre, double *out_lost);
