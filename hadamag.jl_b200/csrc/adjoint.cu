@@ -32,7 +32,7 @@ struct AdjArgs {
   double2 *G;        // chunk x 2^n
   double2 *grad;     // 2^n, accumulated dm/dpsi
   double *mpart;     // per warp: sum (F^2)^q (plain), folded at the end
-  double q, cq_x, cq_0;
+  double q, cq_x, cq_0, q4;
   int n, U, chunk;
   uint64_t x0;  // first X-string (natural order) of the chunk
   int nx;
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(128) k_adj_fused(AdjArgs a) {
 }
 
 // ---------------------------------------------------------------------------------
-// n >= 12.  Pass 1 (forward, low bits) for (x, row); x = 0 uses the zero-pair build.
+// n >= 15.  Pass 1 (forward, low bits) for (x, row); x = 0 uses the zero-pair build.
 template <int HI>
 __global__ void __launch_bounds__(128) k_adj_p1(AdjArgs a) {
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -360,7 +360,139 @@ __global__ void __launch_bounds__(32 * ACC_SEGS) k_adj_acc(AdjArgs a) {
   }
 }
 
-__global__ void k_adj_finish(double2 *grad, uint64_t len, const double *mpart, int nw, double *m_out) {
+// ---------------------------------------------------------------------------------
+// n = 12, 13, 14: one CTA of G = 2^(n-11) warps runs an X-string forward and backward
+// without leaving the SM: the forward half of k_sre_wide (sre_wide.cuh), the pointwise map on
+// the real values of phase B, the same levels again (the WHT is its own transpose), and
+// the exchange back into phase A's layout.  Only Gamma leaves, 2^(n-1) complex per X-string in
+// element order; the four-kernel chain used above moved every X-string through L2 three
+// times more.  Bound: FP64 issue and the exchanges, as the forward kernel, and Gamma's
+// stores (L2 takes 28 bytes per clock and SM).
+template <int G, int QA>
+__global__ void __launch_bounds__(32 * G, 8 / G) k_adj_wide(AdjArgs a) {
+  constexpr uint32_t HALF = 1024u * G;
+  extern __shared__ __align__(128) unsigned char smraw[];
+  double *buf = reinterpret_cast<double *>(smraw);
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t e0 = 1024u * w + lane;
+  double msum = 0.0;
+  for (int xi = blockIdx.x; xi < a.nx; xi += gridDim.x) {
+    const uint32_t x = (uint32_t)a.x0 + xi;
+    double2 v[R];
+    wide_build(v, a.psi, x, e0, HALF);
+    __syncthreads();  // the previous X-string's values have been read
+    wide_put<double, G>(v, buf, w, lane);
+    __syncthreads();
+    wide_get<double, G>(v, buf, w, lane);
+    auto levels = [&] {
+      wide_lane_bits<G>(v, lane);
+#pragma unroll
+      for (int b = 0; b < 8; ++b) wht_block<0, 2>(v, b);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) wht_class<2, 5>(v, c);
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        const double p = v[i].x, q = v[i].y;
+        v[i].x = p + q;
+        v[i].y = p - q;
+      }
+    };
+    levels();
+    const double cq = x == 0 ? a.cq_0 : a.cq_x;
+    double m0 = 0.0, m1 = 0.0;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const double f = v[i].x, g = v[i].y, f2 = f * f, g2 = g * g;
+      const double pf = QA == 2 ? f2 : QA == 3 ? f2 * f2 : powi7(f2, (int)a.q - 1);  // (W^2)^(q-1)
+      const double pg = QA == 2 ? g2 : QA == 3 ? g2 * g2 : powi7(g2, (int)a.q - 1);
+      m0 = fma(pf, f2, m0);
+      m1 = fma(pg, g2, m1);
+      v[i].x = cq * f * pf;
+      v[i].y = cq * g * pg;
+    }
+    msum += (m0 + m1) * (x == 0 ? 1.0 : a.q4);
+    levels();
+    wide_unget<double, G>(v, buf, w, lane);  // each lane's own addresses
+    __syncthreads();
+    wide_unput<double, G>(v, buf, w, lane);
+    double2 *gam = a.G + (size_t)xi * HALF + e0;
+#pragma unroll
+    for (int i = 0; i < R; ++i) __stcg(gam + 32 * i, v[i]);
+  }
+  msum = warp_sum(msum);
+  if (lane == 0) a.mpart[blockIdx.x * G + w] += msum;
+}
+
+// grad(u) += sum over the batch's X-strings of G_x(u) psi(u ^ x), G_x from Gamma_x in element
+// order: with j the highest set bit of x, u or (u's bit j set) u ^ x is the element whose
+// bit j is 0, and dropping that bit gives its place.  Work split and order as k_adj_acc.
+__global__ void __launch_bounds__(32 * ACC_SEGS) k_adj_gather(AdjArgs a) {
+  constexpr int U = 8;  // X-strings' loads in flight per lane
+  __shared__ double2 part[ACC_SEGS][32];
+  const uint32_t len = 1u << a.n, half = len >> 1;
+  const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5;
+  const int per = (a.nx + ACC_SEGS - 1) / ACC_SEGS;
+  const int xb = min(a.nx, seg * per), xe = min(a.nx, xb + per);
+  for (uint32_t base = blockIdx.x * 32u; base < len; base += gridDim.x * 32u) {
+    const uint32_t u = base + lane;
+    double gr[4] = {0.0, 0.0, 0.0, 0.0}, gi[4] = {0.0, 0.0, 0.0, 0.0};
+    // x != 0: Gamma_x at u's place, conjugated when u is the first of the pair
+    auto load = [&](int xi, double2 &g, double2 &p) {
+      const uint32_t x = (uint32_t)a.x0 + xi;
+      const int j = 31 - __clz((int)x);
+      const bool second = (u >> j) & 1;
+      const uint32_t r = second ? u ^ x : u, low = (1u << j) - 1u;
+      g = __ldcg(a.G + (size_t)xi * half + ((r & low) | ((r >> 1) & ~low)));
+      p = __ldg(a.psi + (u ^ x));
+      if (!second) g.y = -g.y;
+    };
+    auto add = [&](const double2 &g, const double2 &p, double &re, double &im) {
+      re += g.x * p.x - g.y * p.y;
+      im += g.x * p.y + g.y * p.x;
+    };
+    int xi = xb;
+    if (a.x0 + xi == 0 && xi < xe) {
+      const double2 g = __ldcg(a.G + (u & (half - 1))), p = __ldg(a.psi + u);
+      const double f = 2.0 * (u < half ? g.x + g.y : g.x - g.y);
+      gr[0] = f * p.x;
+      gi[0] = f * p.y;
+      ++xi;
+    }
+    for (; xi + U <= xe; xi += U) {
+      double2 g[U], p[U];
+#pragma unroll
+      for (int k = 0; k < U; ++k) load(xi + k, g[k], p[k]);
+#pragma unroll
+      for (int k = 0; k < U; ++k) add(g[k], p[k], gr[k & 3], gi[k & 3]);
+    }
+    for (; xi < xe; ++xi) {
+      double2 g, p;
+      load(xi, g, p);
+      add(g, p, gr[0], gi[0]);
+    }
+    part[seg][lane] = make_double2((gr[0] + gr[1]) + (gr[2] + gr[3]), (gi[0] + gi[1]) + (gi[2] + gi[3]));
+    __syncthreads();
+    if (seg == 0) {
+      double2 sum = part[0][lane];
+#pragma unroll
+      for (int k = 1; k < ACC_SEGS; ++k) {
+        sum.x += part[k][lane].x;
+        sum.y += part[k][lane].y;
+      }
+      double2 o = a.grad[u];
+      o.x += sum.x;
+      o.y += sum.y;
+      a.grad[u] = o;
+    }
+    __syncthreads();
+  }
+}
+
+// Every block adds up the moment partials in the same order (so all hold the same m), then
+// scales its part of the gradient: one block alone took 57 us at n = 14 and four times that
+// for every two qubits more.
+__global__ void __launch_bounds__(256) k_adj_finish(double2 *grad, uint64_t len, const double *mpart, int nw,
+                                                    double *m_out) {
   __shared__ double sh[256];
   double s = 0.0;
   for (int i = threadIdx.x; i < nw; i += blockDim.x) s += mpart[i];
@@ -372,16 +504,15 @@ __global__ void k_adj_finish(double2 *grad, uint64_t len, const double *mpart, i
   }
   const double m = sh[0];
   const double scale = -1.0 / (m * 0.69314718055994530942);
-  for (uint64_t i = threadIdx.x; i < len; i += blockDim.x) {
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < len; i += (uint64_t)gridDim.x * blockDim.x) {
     double2 g = grad[i];
     grad[i] = make_double2(g.x * scale, g.y * scale);
   }
-  if (threadIdx.x == 0) *m_out = m;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *m_out = m;
 }
 
-
 // ---------------------------------------------------------------------------------
-// n >= 12, X-strings x >= 2^PB: stage kernels.  Batch b holds the X consecutive
+// n >= 15, X-strings x >= 2^PB: stage kernels.  Batch b holds the X consecutive
 // X-strings x_begin + b X + xs (aligned, so they share their pairing bit and the rows
 // rH, sH of every rho; only the low bits xs of x differ).  Stage t runs four kernels,
 // one per kind of unit (independent work inside the stage):
@@ -765,9 +896,6 @@ int run_adj_stages(hm_ctx *c, const double2 *psi, int n, int q, double2 *grad, d
     r = q == 2 ? launch_adj_stages<HIv, 2>(c, a, nw)                                     \
                : (q == 3 ? launch_adj_stages<HIv, 3>(c, a, nw) : launch_adj_stages<HIv, 0>(c, a, nw)); \
     break;
-    HM_ADJS(1)
-    HM_ADJS(2)
-    HM_ADJS(3)
     HM_ADJS(4)
     HM_ADJS(5)
     HM_ADJS(6)
@@ -789,6 +917,65 @@ int run_adj_stages(hm_ctx *c, const double2 *psi, int n, int q, double2 *grad, d
 
 }  // namespace
 
+// scale the gradient by -1 / (m ln 2) and read m back
+static int adj_results(hm_ctx *c, double2 *grad_dev, uint64_t len, const double *mpart, int nslots, double *m_out) {
+  HM_CUDA(c, cudaEventRecord(c->ev1, c->stream));
+  HM_TRY(ensure_dev(c, (void **)&c->d_out, &c->out_cap, sizeof(double) * 16));
+  k_adj_finish<<<(unsigned)std::max<uint64_t>(1, std::min<uint64_t>(len / 256, 2 * (uint64_t)c->num_sms)), 256, 0,
+                 c->stream>>>(grad_dev, len, mpart, nslots, c->d_out);
+  c->launches += 1;
+  HM_TRY(ensure_host(c, (void **)&c->h_out, &c->h_out_cap, sizeof(double) * 24));
+  HM_CUDA(c, cudaMemcpyAsync(c->h_out, c->d_out, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  HM_CUDA(c, cudaStreamSynchronize(c->stream));
+  float ms = 0.f;
+  HM_CUDA(c, cudaEventElapsedTime(&ms, c->ev0, c->ev1));
+  c->last_ms = ms;
+  *m_out = c->h_out[0];
+  return HM_OK;
+}
+
+// n = 12, 13, 14: batches of whole rounds of k_adj_wide's CTAs, each followed by its share of
+// the gradient.  Three rounds make 57 MB of Gamma, which the gather finds in L2: n = 14
+// 2.05 ms of kernels; with two rounds 2.28 (more launches), with four 2.26 (Gamma leaves
+// L2).  The four-kernel stages took 2.68 (n = 12: 0.27 -> 0.22, n = 13: 0.78 -> 0.60).
+static constexpr int wide_rounds = 3;
+
+template <int G>
+static int launch_adj_wide(hm_ctx *c, AdjArgs &a, double *m_out, double2 *grad_dev) {
+  const uint64_t len = 2048ull * G;
+  const size_t smem = 2048 * G * sizeof(double);
+  auto kern = a.q == 2.0 ? k_adj_wide<G, 2> : a.q == 3.0 ? k_adj_wide<G, 3> : k_adj_wide<G, 0>;
+  int occ = 0;
+  HM_TRY(kernel_occ(c, kern, 32 * G, smem, &occ));
+  const int blocks = (int)std::min<uint64_t>(len, (uint64_t)c->num_sms * occ), nslots = blocks * G;
+  const int batch = (int)std::min<uint64_t>(len, (uint64_t)wide_rounds * blocks);
+  HM_TRY(ensure_dev(c, &c->d_inter, &c->inter_cap, (size_t)batch * (len / 2) * sizeof(double2)));
+  a.G = (double2 *)c->d_inter;
+  a.grad = grad_dev;
+  HM_CUDA(c, cudaMemsetAsync(grad_dev, 0, len * sizeof(double2), c->stream));
+  HM_TRY(ensure_dev(c, (void **)&c->d_partials, &c->partials_cap, nslots * sizeof(double)));
+  HM_CUDA(c, cudaMemsetAsync(c->d_partials, 0, nslots * sizeof(double), c->stream));
+  a.mpart = c->d_partials;
+  HM_CUDA(c, cudaEventRecord(c->ev0, c->stream));
+  for (uint64_t x0 = 0; x0 < len; x0 += batch) {
+    a.x0 = x0;
+    a.nx = (int)std::min<uint64_t>(batch, len - x0);
+    kern<<<std::min(blocks, a.nx), 32 * G, smem, c->stream>>>(a);
+    k_adj_gather<<<(unsigned)(len / 32), 32 * ACC_SEGS, 0, c->stream>>>(a);
+    c->launches += 2;
+  }
+  HM_CUDA(c, cudaGetLastError());
+  return adj_results(c, grad_dev, len, a.mpart, nslots, m_out);
+}
+
+static int run_adj_wide(hm_ctx *c, AdjArgs &a, double *m_out, double2 *grad_dev) {
+  switch (a.n) {
+    case 12: return launch_adj_wide<2>(c, a, m_out, grad_dev);
+    case 13: return launch_adj_wide<4>(c, a, m_out, grad_dev);
+    default: return launch_adj_wide<8>(c, a, m_out, grad_dev);
+  }
+}
+
 int run_sre_grad(hm_ctx *c, const double2 *psi, int n, int q, double *m_out, double2 *grad_dev) {
   AdjArgs a;
   memset(&a, 0, sizeof a);
@@ -797,7 +984,9 @@ int run_sre_grad(hm_ctx *c, const double2 *psi, int n, int q, double *m_out, dou
   a.q = q;
   a.cq_x = 2.0 * q * pow(4.0, q);
   a.cq_0 = 2.0 * q;
+  a.q4 = pow(4.0, q);
   const uint64_t len = 1ull << n;
+  if (n >= 12 && n <= 14) return run_adj_wide(c, a, m_out, grad_dev);
   // chunk: G of at most 1 GiB.  Each chunk costs four launches; with small chunks (16
   // X-strings at n = 18 for 64 MiB) the launches were under-filled and dominated the time
   int chunk = (int)std::max<uint64_t>(1, ((uint64_t)1 << 30) / (len * sizeof(double2)));
@@ -805,7 +994,7 @@ int run_sre_grad(hm_ctx *c, const double2 *psi, int n, int q, double *m_out, dou
   if (n >= 12 && chunk > (1 << PB)) chunk = 1 << PB;  // the chunked kernels only see x < 2^PB
   a.chunk = chunk;
   HM_TRY(ensure_dev(c, &c->d_inter, &c->inter_cap, (size_t)chunk * len * sizeof(double2) +
-                                                       (n >= 12 ? (size_t)chunk * (len / 2) * sizeof(double2) : 0)));
+                                                       (n >= 15 ? (size_t)chunk * (len / 2) * sizeof(double2) : 0)));
   a.G = (double2 *)c->d_inter;
   a.ring = a.G + (size_t)chunk * len;
   a.grad = grad_dev;
@@ -869,9 +1058,6 @@ int run_sre_grad(hm_ctx *c, const double2 *psi, int n, int q, double *m_out, dou
     k_adj_p1b<HIv><<<blocks, 128, smem, c->stream>>>(a);                                          \
     break;
       switch (n - 11) {
-        HM_ADJP(1)
-        HM_ADJP(2)
-        HM_ADJP(3)
         HM_ADJP(4)
         HM_ADJP(5)
         HM_ADJP(6)
@@ -892,18 +1078,7 @@ int run_sre_grad(hm_ctx *c, const double2 *psi, int n, int q, double *m_out, dou
     int nw_st = 0;
     HM_TRY(run_adj_stages(c, psi, n, q, grad_dev, c->d_partials + nw, &nw_st));
   }
-  HM_CUDA(c, cudaEventRecord(c->ev1, c->stream));
-  HM_TRY(ensure_dev(c, (void **)&c->d_out, &c->out_cap, sizeof(double) * 16));
-  k_adj_finish<<<1, 256, 0, c->stream>>>(grad_dev, len, a.mpart, (int)nslots, c->d_out);
-  c->launches += 1;
-  HM_TRY(ensure_host(c, (void **)&c->h_out, &c->h_out_cap, sizeof(double) * 24));
-  HM_CUDA(c, cudaMemcpyAsync(c->h_out, c->d_out, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  HM_CUDA(c, cudaStreamSynchronize(c->stream));
-  float ms = 0.f;
-  HM_CUDA(c, cudaEventElapsedTime(&ms, c->ev0, c->ev1));
-  c->last_ms = ms;
-  *m_out = c->h_out[0];
-  return HM_OK;
+  return adj_results(c, grad_dev, len, a.mpart, (int)nslots, m_out);
 }
 
 }  // namespace hm

@@ -133,6 +133,36 @@ __device__ __forceinline__ void wide_get(V (&v)[32], const T *buf, int w, int la
   }
 }
 
+// wide_get and wide_put the other way, for a backward transform: phase B's values into the
+// planes (each lane's own addresses), and the planes into phase A's registers with the
+// butterflies over bits 5 .. 9
+template <typename T, int G, typename V>
+__device__ __forceinline__ void wide_unget(const V (&v)[32], T *buf, int w, int lane) {
+  static_assert(sizeof(T) == 8, "FP64 only");
+  T *plane = buf + (w >= G / 2 ? 1024 * G : 0);
+  const uint32_t base = wide_base<G>(w, lane);
+#pragma unroll
+  for (int b = 0; b < 2; ++b)
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      *reinterpret_cast<V *>(plane + wide_pos<T, G>(base | (2 * i)) + 1024 * b) = v[16 * b + i];
+}
+template <typename T, int G, typename V>
+__device__ __forceinline__ void wide_unput(V (&v)[32], const T *buf, int w, int lane) {
+#pragma unroll
+  for (int b = 0; b < 8; ++b) {
+#pragma unroll
+    for (int i = 4 * b; i < 4 * b + 4; ++i) {
+      const uint32_t p = wide_pos<T, G>((uint32_t)(32 * i + lane) + 1024u * w);
+      v[i].x = buf[p];
+      v[i].y = buf[1024 * G + p];
+    }
+    wht_block<0, 2>(v, b);
+  }
+#pragma unroll
+  for (int c = 0; c < 4; ++c) wht_class<2, 5>(v, c);
+}
+
 // one transform bit held by lane bit `m` (a mask): every value meets its partner's
 template <typename V>
 __device__ __forceinline__ void lane_wht(V (&v)[32], int lane, int m) {

@@ -56,3 +56,12 @@ def test_two_pass_ranges(ctx, hm, n, qs, precision):
         for p, v in ((p2, m), (p2s, ms)):
             assert p.sum() == pytest.approx(p2r.sum(), rel=tol)
             assert v.sum(axis=1) == pytest.approx(mr.sum(axis=1), rel=tol)
+
+
+@pytest.mark.parametrize("n,q", [(12, 4), (13, 1), (13, 3), (14, 8)])
+def test_grad_single_cta(ctx, oracle, n, q):
+    psi = rand_state(1 << n, 950 + n)
+    v, g = ctx.sre_grad(psi, q)
+    ov, og = oracle.sre_grad(psi, q)
+    assert abs(v - ov) <= 1e-10 * max(1.0, abs(ov))  # q = 1: the value is 0 up to rounding
+    assert abs(g - og).max() <= 1e-10 * abs(og).max()
