@@ -7,6 +7,11 @@
 // is log2(S) / log2(3).  The sum over x does not depend on the order in which the
 // X-strings are visited, so x runs over 0 .. 3^L - 1 directly.
 //
+// v(-r) = conj v(r), so W is real, and two X-strings share one complex transform:
+// v_1 + i v_2 transforms into W_1 + i W_2, whose parts give |W_1| + |W_2| without a square
+// root.  That halves the transforms, the intermediate's traffic and the launches (B200, whole
+// call: L = 8 0.71 -> 0.36 ms, 9 4.70 -> 2.37, 10 42.9 -> 22.0, 11 368 -> 196).
+//
 // The 3^L-point transform is split like the exact-SRE sweep: the low `lo` digits of r
 // form a contiguous row (pass 1: gather + build + transform in shared memory), the high
 // `hi` digits a strided column (pass 2: transform + sum |W|).  Batches of X-strings keep
@@ -109,7 +114,11 @@ __device__ __forceinline__ void h3_regs(double2 (&v)[NREG]) {
   if constexpr (ND >= 3) h3_digit<NREG, 9>(v);
 }
 
-constexpr int MANA_MAX_THREADS = 256;
+// Threads per CTA, and CTAs per SM of the two passes: pass 1 keeps 27 complex values (108
+// registers) while it adds a second X-string to them, and spills below 255 registers (two
+// CTAs; L = 9 2.37 ms per call, three with 184 B of spills 2.46); pass 2 needs registers for
+// its 27 loads in flight (three CTAs; four at 128 registers 2.85).
+constexpr int MANA_MAX_THREADS = 128, MANA_CTAS1 = 2, MANA_CTAS2 = 3;
 
 // shape of the two-pass split for L = LO + HI qutrits: pass 1 transforms rows of
 // RL = 3^LO elements (ROWS rows per CTA), pass 2 columns of RH = 3^HI elements (COLS
@@ -134,12 +143,15 @@ struct ManaArgs {
   const double2 *psi;
   double2 *inter;  // batch x RH x RL
   double *slots;   // per pass-2 CTA slot: dd (2 doubles)
-  int x0, nx;      // X-strings of this batch: x0 .. x0 + nx - 1
+  int x0, nx;      // first X-strings of this batch's pairs: x0 .. x0 + nx - 1
+  int xs, xe;      // the partner of x is x + xs, if below xe (xs: a multiple of RL)
   double invdim;
 };
 
-// pass 1: rows [blockIdx.x * ROWS, ...) of X-string x0 + blockIdx.y: gather + build
-// v(r) = conj psi(r (+) x) psi((-r) (+) x) / 3^L, transform the row digits.  Pass 1 runs
+// pass 1: rows [blockIdx.x * ROWS, ...) of the pair x, x + xs with x = x0 + blockIdx.y:
+// gather + build v_1 + i v_2, v(r) = conj psi(r (+) x) psi((-r) (+) x) (the factor 1 / 3^L is
+// applied to the sums), transform the row digits.  The partners share their row digits xL,
+// so only the row pointers differ.  Pass 1 runs
 // the block phases in the other order: phase A takes the HIGH three digits, thread t
 // holding e = t + T k (so a warp's gathers for one k are adjacent elements), and phase B
 // the low B digits in contiguous groups, thread t holding e = m + MB (t + T s).  The row
@@ -147,7 +159,7 @@ struct ManaArgs {
 // a fixed permutation of the positions, which pass 2 (columns) and the sum of |W| do not
 // see, and which makes every store instruction of a warp contiguous.
 template <int LO, int HI>
-__global__ void __launch_bounds__(MANA_MAX_THREADS, 2) k_mana_p1(ManaArgs a) {
+__global__ void __launch_bounds__(MANA_MAX_THREADS, MANA_CTAS1) k_mana_p1(ManaArgs a) {
   using S = ManaShape<LO, HI>;
   using Q = typename S::QR;
   constexpr int RL = S::RL, RH = S::RH, ROWS = S::ROWS, E = Q::E, T = Q::T;
@@ -162,6 +174,7 @@ __global__ void __launch_bounds__(MANA_MAX_THREADS, 2) k_mana_p1(ManaArgs a) {
   }
   const int x = a.x0 + xi;
   const int xL = x % RL, xH = x / RL;
+  const bool two = x + a.xs < a.xe;  // uniform across the CTA
   const int row0 = blockIdx.x * ROWS;
   const int nrows = min(ROWS, RH - row0);
   const int rr = threadIdx.x / T, t = threadIdx.x - rr * T;
@@ -169,33 +182,49 @@ __global__ void __launch_bounds__(MANA_MAX_THREADS, 2) k_mana_p1(ManaArgs a) {
   double2 v[E];
   if (act) {
     const int row = row0 + rr;
-    const double2 *pa = a.psi + (size_t)tadd(row, xH, HI) * RL;
-    const double2 *pb = a.psi + (size_t)tnegadd(row, xH, HI) * RL;
     // e = t + T k: the digit-wise e (+) xL and (-e) (+) xL split into the low B digits
     // (t, once per thread) and the A register digits of k, whose rotations by the digits
-    // of xL are picked per register at compile time (no table, no shared-memory load)
+    // of xL are picked per register at compile time (no table, no shared-memory load);
+    // the rotation of -c is that of 3 - c
     const int xlo = xL % T, xhi = xL / T;
-    const int at = tadd(t, xlo, Q::B), nt = tnegadd(t, xlo, Q::B);
-    int ra[3][3], rn[3][3];
+    const double2 *pa = a.psi + (size_t)tadd(row, xH, HI) * RL + tadd(t, xlo, Q::B);
+    const double2 *pb = a.psi + (size_t)tnegadd(row, xH, HI) * RL + tnegadd(t, xlo, Q::B);
+    int ra[3][3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
       const int h = (xhi / ipow3c(i)) % 3;
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        ra[i][c] = ((h + c) % 3) * ipow3c(i) * T;
-        rn[i][c] = ((h + 3 - c) % 3) * ipow3c(i) * T;
-      }
+      for (int c = 0; c < 3; ++c) ra[i][c] = ((h + c) % 3) * ipow3c(i) * T;
     }
+    auto ia = [&](int k) {
+      return ra[0][k % 3] + (Q::A > 1 ? ra[1][(k / 3) % 3] : 0) + (Q::A > 2 ? ra[2][k / 9] : 0);
+    };
+    auto in = [&](int k) {
+      return ra[0][(3 - k % 3) % 3] + (Q::A > 1 ? ra[1][(3 - (k / 3) % 3) % 3] : 0) +
+             (Q::A > 2 ? ra[2][(3 - k / 9) % 3] : 0);
+    };
+    if (two) {
+      const int xH2 = (x + a.xs) / RL;
+      const double2 *pc = a.psi + (size_t)tadd(row, xH2, HI) * RL + tadd(t, xlo, Q::B);
+      const double2 *pd = a.psi + (size_t)tnegadd(row, xH2, HI) * RL + tnegadd(t, xlo, Q::B);
+      // v = conj(p) q + i conj(u) w, one X-string after the other (fewer loads to hold)
 #pragma unroll
-    for (int k = 0; k < E; ++k) {
-      const int k0 = k % 3, k1 = (k / 3) % 3, k2 = (k / 9) % 3;
-      const int ia = at + ra[0][k0] + (Q::A > 1 ? ra[1][k1] : 0) + (Q::A > 2 ? ra[2][k2] : 0);
-      const int in = nt + rn[0][k0] + (Q::A > 1 ? rn[1][k1] : 0) + (Q::A > 2 ? rn[2][k2] : 0);
-      const double2 p = pa[ia];
-      double2 q = pb[in];
-      q.x *= a.invdim;
-      q.y *= a.invdim;
-      v[k] = make_double2(p.x * q.x + p.y * q.y, p.x * q.y - p.y * q.x);  // conj(p) * q
+      for (int k = 0; k < E; ++k) {
+        const double2 p = pa[ia(k)], q = pb[in(k)];
+        v[k] = make_double2(fma(p.x, q.x, p.y * q.y), fma(p.x, q.y, -(p.y * q.x)));
+      }
+#pragma unroll
+      for (int k = 0; k < E; ++k) {
+        const double2 u = pc[ia(k)], w = pd[in(k)];
+        v[k].x = fma(u.y, w.x, fma(-u.x, w.y, v[k].x));
+        v[k].y = fma(u.x, w.x, fma(u.y, w.y, v[k].y));
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < E; ++k) {
+        const double2 p = pa[ia(k)], q = pb[in(k)];
+        v[k] = make_double2(fma(p.x, q.x, p.y * q.y), fma(p.x, q.y, -(p.y * q.x)));
+      }
     }
     h3_regs<E, Q::A>(v);  // the register digits of k: element digits B .. LO-1
   }
@@ -227,10 +256,11 @@ __global__ void __launch_bounds__(MANA_MAX_THREADS, 2) k_mana_p1(ManaArgs a) {
   }
 }
 
-// pass 2: columns [blockIdx.x * COLS, ...) of X-string x0 + blockIdx.y: transform the
-// column digits and add the CTA's sum |W| into its double-double slot
+// pass 2: columns [blockIdx.x * COLS, ...) of the pair blockIdx.y: transform the column
+// digits and add the CTA's sum |W_1| + |W_2| (the second is 0 without a partner, whose
+// imaginary parts are rounding errors) into its double-double slot
 template <int LO, int HI>
-__global__ void __launch_bounds__(MANA_MAX_THREADS, 2) k_mana_p2(ManaArgs a) {
+__global__ void __launch_bounds__(MANA_MAX_THREADS, MANA_CTAS2) k_mana_p2(ManaArgs a) {
   using S = ManaShape<LO, HI>;
   using Q = typename S::QC;
   constexpr int RL = S::RL, RH = S::RH, COLS = S::COLS, E = Q::E, T = Q::T;
@@ -242,6 +272,7 @@ __global__ void __launch_bounds__(MANA_MAX_THREADS, 2) k_mana_p2(ManaArgs a) {
   const int ncols = min(COLS, RL - c0);
   const int t = threadIdx.x / COLS, c = threadIdx.x - t * COLS;
   const bool act = xi < a.nx && t < T && c < ncols;
+  const bool two = a.x0 + xi + a.xs < a.xe;
   const double2 *in = a.inter + (size_t)xi * RH * RL + c0 + c;
   double2 v[E];
   mana_allow_next();
@@ -268,7 +299,8 @@ __global__ void __launch_bounds__(MANA_MAX_THREADS, 2) k_mana_p2(ManaArgs a) {
   double sum = 0.0;
   if (act) {
 #pragma unroll
-    for (int k = 0; k < E; ++k) sum += sqrt(fma(v[k].x, v[k].x, v[k].y * v[k].y));
+    for (int k = 0; k < E; ++k) sum += fabs(v[k].x) + (two ? fabs(v[k].y) : 0.0);
+    sum *= a.invdim;
   }
   // warp sums, then the warps' sums in warp order
   sum = warp_sum(sum);
@@ -468,8 +500,12 @@ static int run_mana_pure_t(hm_ctx *c, const double2 *psi, int xb, int xe, double
   const int bmax = (int)std::max<size_t>(1, ((size_t)64 << 20) / per_x);
   int B = std::min(bmax, std::max(1, wave / g1));
   for (int w = 2; (long long)w * wave / g1 <= bmax; ++w) B = (int)((long long)w * wave / g1);
-  if (B > xe - xb) B = xe - xb;
-  if (B > D) B = D;
+  // partners: x and x + xs, xs the multiple of RL that covers half of the range
+  const int n = xe - xb, halves = (n + 2 * S::RL - 1) / (2 * S::RL);
+  a.xs = halves * S::RL;
+  a.xe = xe;
+  const int npair = std::min(n, a.xs);
+  if (B > npair) B = npair;
   HM_TRY(ensure_dev(c, &c->d_inter, &c->inter_cap, (size_t)B * per_x));
   a.inter = (double2 *)c->d_inter;
   const size_t nslots = (size_t)g2 * B;
@@ -477,9 +513,9 @@ static int run_mana_pure_t(hm_ctx *c, const double2 *psi, int xb, int xe, double
   HM_CUDA(c, cudaMemsetAsync(c->d_partials, 0, nslots * 2 * sizeof(double), c->stream));
   a.slots = c->d_partials;
   HM_CUDA(c, cudaEventRecord(c->ev0, c->stream));
-  for (int x0 = xb; x0 < xe; x0 += B) {
+  for (int x0 = xb; x0 < xb + npair; x0 += B) {
     a.x0 = x0;
-    a.nx = std::min(B, xe - x0);
+    a.nx = std::min(B, xb + npair - x0);
     HM_TRY(mana_launch(c, k1, dim3(g1, a.nx), S::NT1, S::SM1, a, x0 > xb));
     HM_TRY(mana_launch(c, k2, dim3(g2, B), S::NT2, S::SM2, a, true));
     c->launches += 2;

@@ -65,3 +65,13 @@ def test_grad_single_cta(ctx, oracle, n, q):
     ov, og = oracle.sre_grad(psi, q)
     assert abs(v - ov) <= 1e-10 * max(1.0, abs(ov))  # q = 1: the value is 0 up to rounding
     assert abs(g - og).max() <= 1e-10 * abs(og).max()
+
+
+@pytest.mark.parametrize("L", [1, 2, 3, 5, 7, 8])
+def test_mana_pairs_equal_single_x_strings(ctx, L):
+    # X-strings of a range share transforms in pairs; a range of one has no partner
+    psi, D = rand_state(3 ** L, 970 + L), 3 ** L
+    for a, b in {(0, D), (D // 3, D), (max(0, D - 41), D)}:
+        if b - a <= 300:
+            singles = sum(ctx.mana_pure_range(psi, x, x + 1).sum() for x in range(a, b))
+            assert ctx.mana_pure_range(psi, a, b).sum() == pytest.approx(singles, rel=1e-13)
