@@ -86,6 +86,159 @@ int launch_2gate(hm_ctx *c, double2 *psi, int n, int q, const double *gate_colma
 }
 
 // ---------------------------------------------------------------------------------
+// Brick walls.  One launch per gate passes the whole state through L2 for 4 (q = 2) complex
+// multiply-adds per amplitude.  Instead a pass takes a window of adjacent sites into shared
+// memory, up to TS amplitudes per CTA, and applies every gate of the circuit that lies inside the
+// window and whose earlier gates on the same sites have been applied (the host picks the
+// window that advances most gates; at n = 18, depth 8, the 68 gates take five passes).  A
+// window above site 1 also holds the lowest C sites, so that the tile's runs in memory are
+// q^C amplitudes (64 or 144 bytes).  The arithmetic of a gate is that of k_apply_2gate.
+template <int Q> struct Window {
+  static constexpr int SITES = Q == 2 ? 12 : 7, C = 2;  // sites of a tile; of them low sites
+  static constexpr int TS = Q == 2 ? 4096 : 2187;
+  static constexpr size_t SMEM = (TS + 7) / 8 * 8 * sizeof(double2);  // win_sw stays inside eights
+};
+constexpr int WINDOW_GATES = 256;
+
+struct GateList {
+  int n;                        // gates of this pass
+  unsigned short gate[WINDOW_GATES];  // index into the gate array, from the pass's first gate
+  unsigned char pos[WINDOW_GATES];    // tile position of the gate's lower site
+};
+
+// 16-byte granules of a 128-byte bank row XOR-ed with higher index bits
+__device__ __forceinline__ int win_sw(int i) { return i ^ ((i >> 3) & 7) ^ ((i >> 6) & 7); }
+
+// tile = low + q^c (m + q^w (window digits above)) with c low sites and w window sites:
+// ts = q^(c+w) amplitudes; amplitude i of tile t sits at
+//   (i mod q^c) + q^c (t mod ql) + q^w0 (i div q^c) + q^(w0+w) (t div ql),  ql = q^(w0-c)
+template <int Q>
+__global__ void __launch_bounds__(256) k_gate_window(double2 *__restrict__ psi, const double2 *__restrict__ gates,
+                                                     uint64_t ntiles, int ts, int qc, uint64_t ql, uint64_t qw0,
+                                                     uint64_t qtop, const __grid_constant__ GateList list) {
+  constexpr int Q2 = Q * Q, Q4 = Q2 * Q2;
+  extern __shared__ __align__(128) unsigned char smraw[];
+  double2 *tile = reinterpret_cast<double2 *>(smraw);
+  __shared__ double2 G[2][Q4];  // column-major: G[in Q2 + o]
+  for (uint64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    double2 *base = psi + (uint64_t)qc * (t % ql) + qtop * (t / ql);
+    for (int i = threadIdx.x; i < ts; i += blockDim.x) tile[win_sw(i)] = base[i % qc + qw0 * (uint64_t)(i / qc)];
+    if (threadIdx.x < Q4) G[0][threadIdx.x] = gates[(size_t)list.gate[0] * Q4 + threadIdx.x];
+    __syncthreads();
+    for (int k = 0; k < list.n; ++k) {
+      const double2 *g = G[k & 1];
+      if (k + 1 < list.n && threadIdx.x < Q4)
+        G[(k + 1) & 1][threadIdx.x] = gates[(size_t)list.gate[k + 1] * Q4 + threadIdx.x];
+      int p1 = 1;
+      for (int d = 0; d < list.pos[k]; ++d) p1 *= Q;
+      const int p2 = p1 * Q;
+      for (int u = threadIdx.x; u < ts / Q2; u += blockDim.x) {
+        const int b = u % p1 + p1 * Q2 * (u / p1);
+        double2 a[Q2];
+#pragma unroll
+        for (int in = 0; in < Q2; ++in) a[in] = tile[win_sw(b + (in / Q) * p1 + (in % Q) * p2)];
+#pragma unroll(Q == 2 ? Q2 : 1)  // q = 3: its 81 entries do not fit the registers
+        for (int o = 0; o < Q2; ++o) {
+          double re = 0.0, im = 0.0;
+#pragma unroll
+          for (int in = 0; in < Q2; ++in) {
+            const double2 c = g[in * Q2 + o];
+            re = fma(c.x, a[in].x, fma(-c.y, a[in].y, re));
+            im = fma(c.x, a[in].y, fma(c.y, a[in].x, im));
+          }
+          tile[win_sw(b + (o / Q) * p1 + (o % Q) * p2)] = make_double2(re, im);
+        }
+      }
+      __syncthreads();
+    }
+    for (int i = threadIdx.x; i < ts; i += blockDim.x) base[i % qc + qw0 * (uint64_t)(i / qc)] = tile[win_sw(i)];
+    __syncthreads();
+  }
+}
+
+// The gates of `order` (indices of gates not yet applied, first site in site[], 0-based) that
+// a window over sites [w0, w0 + w) can apply now, in order.
+void window_take(const std::vector<int> &order, const std::vector<int> &site, int n, int w0, int w,
+                 std::vector<int> &take) {
+  take.clear();
+  std::vector<char> blocked(n, 0);
+  int open = n;
+  for (int g : order) {
+    const int s = site[g];
+    if (!blocked[s] && !blocked[s + 1] && s >= w0 && s + 1 < w0 + w && (int)take.size() < WINDOW_GATES &&
+        (take.empty() || g - take[0] < 65536)) {
+      take.push_back(g);
+    } else {
+      open -= !blocked[s];
+      open -= !blocked[s + 1];
+      blocked[s] = blocked[s + 1] = 1;
+      if (open <= 1) break;
+    }
+  }
+}
+
+// Sites of a tile, at most Window<Q>::SITES: smaller tiles occupy more SMs (the gates' FP64
+// work bounds a pass), larger ones save passes.  us for depth 8 on B200, one launch per gate
+// -> this: q = 2 n = 10 191 -> 40, n = 12 181 -> 42 (12 sites: 76), n = 16 249 -> 68 (12: 115),
+// n = 18 282 -> 85 (11: 94, 12: 128), n = 19 365 -> 136, n = 20 490 -> 219 (11: 263, 10: 321);
+// q = 3 n = 7 126 -> 58, n = 10 194 -> 100 (7 sites: 116), n = 12 372 -> 198 (6: 267).
+template <int Q>
+int window_sites(int n) {
+  if (Q == 2) return n <= 13 ? 9 : n <= 18 ? 10 : n == 19 ? 11 : 12;
+  return n >= 8 && n <= 10 ? 6 : 7;
+}
+
+template <int Q>
+int run_brick_wall(hm_ctx *c, double2 *psi, int n, const double2 *gates_dev, const std::vector<int> &site) {
+  using W = Window<Q>;
+  std::vector<int> order(site.size()), take, best;
+  for (size_t i = 0; i < site.size(); ++i) order[i] = (int)i;
+  const int sites = window_sites<Q>(n);
+  const int wlow = n < sites ? n : sites;  // window at the lowest site: the whole tile
+  while (!order.empty()) {
+    int bw = 0;
+    best.clear();
+    for (int w0 = 0; w0 + 1 < n; ++w0) {
+      if (w0 > 0 && (w0 < W::C || w0 + (sites - W::C) > n)) continue;
+      window_take(order, site, n, w0, w0 ? sites - W::C : wlow, take);
+      if (take.size() > best.size()) {
+        best.swap(take);
+        bw = w0;
+      }
+    }
+    const int cs = bw ? W::C : 0, w = bw ? sites - W::C : wlow;
+    GateList list;
+    list.n = (int)best.size();
+    for (int k = 0; k < list.n; ++k) {
+      list.gate[k] = (unsigned short)(best[k] - best[0]);
+      list.pos[k] = (unsigned char)(cs + site[best[k]] - bw);
+    }
+    const double2 *gbase = gates_dev + (size_t)best[0] * (Q * Q * Q * Q);
+    const uint64_t N = upow(Q, n);
+    const int ts = (int)upow(Q, cs + w);
+    auto kern = k_gate_window<Q>;
+    int occ = 0;
+    HM_TRY(kernel_occ(c, kern, 256, W::SMEM, &occ));
+    const uint64_t ntiles = N / ts;
+    const unsigned blocks = (unsigned)std::min<uint64_t>(ntiles, (uint64_t)c->num_sms * occ);
+    kern<<<blocks, 256, W::SMEM, c->stream>>>(
+        psi, gbase, ntiles, ts, (int)upow(Q, cs), bw ? upow(Q, bw - cs) : 1, bw ? upow(Q, bw) : 1, upow(Q, bw + w), list);
+    c->launches += 1;
+    HM_CUDA(c, cudaGetLastError());
+    // what is left, in order
+    size_t j = 0, o = 0;
+    for (size_t i = 0; i < order.size(); ++i) {
+      if (j < best.size() && order[i] == best[j])
+        ++j;
+      else
+        order[o++] = order[i];
+    }
+    order.resize(o);
+  }
+  return HM_OK;
+}
+
+// ---------------------------------------------------------------------------------
 // rho_A[i, j] = sum_k A(i, k) conj(A(j, k)),  A(i, k) = psi[i + dimA k] (left) or
 // psi[i dimB + k] (right); column-major output.  64 x 64 output tiles, 256 threads with
 // 4 x 4 outputs each (16 complex multiply-adds per 8 shared-memory loads), k in slices
@@ -208,13 +361,18 @@ int hm_brick_wall(hm_ctx *c, double *psi, int n, int q, int depth, const double 
   c->launches = 0;
   const size_t bytes = hm::upow(q, n) * sizeof(double2);
   const int q4 = q * q * q * q;
+  const size_t gbytes = (size_t)ngates * q4 * sizeof(double2);
   HM_TRY(hm::ensure_dev(c, &c->d_psi, &c->psi_cap, bytes));
+  HM_TRY(hm::ensure_dev(c, &c->d_aux, &c->aux_cap, gbytes));
   HM_CUDA(c, cudaMemcpyAsync(c->d_psi, psi, bytes, cudaMemcpyHostToDevice, c->stream));
+  if (ngates > 0) HM_CUDA(c, cudaMemcpyAsync(c->d_aux, gates, gbytes, cudaMemcpyHostToDevice, c->stream));
   HM_CUDA(c, cudaEventRecord(c->ev0, c->stream));
-  int k = 0;
+  std::vector<int> site;
+  site.reserve(ngates);
   for (int layer = 1; layer <= depth; ++layer)
-    for (int s = (layer & 1) ? 1 : 2; s <= n - 1; s += 2, ++k)
-      HM_TRY(hm::launch_2gate(c, (double2 *)c->d_psi, n, q, gates + (size_t)2 * q4 * k, s, s + 1));
+    for (int s = (layer & 1) ? 1 : 2; s <= n - 1; s += 2) site.push_back(s - 1);
+  HM_TRY(q == 2 ? hm::run_brick_wall<2>(c, (double2 *)c->d_psi, n, (const double2 *)c->d_aux, site)
+                : hm::run_brick_wall<3>(c, (double2 *)c->d_psi, n, (const double2 *)c->d_aux, site));
   HM_CUDA(c, cudaEventRecord(c->ev1, c->stream));
   HM_CUDA(c, cudaMemcpyAsync(psi, c->d_psi, bytes, cudaMemcpyDeviceToHost, c->stream));
   HM_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -236,10 +394,11 @@ int hm_reduced_density_matrix(hm_ctx *c, const double *psi, int n, int q, int NA
   HM_CUDA(c, cudaSetDevice(c->device));
   c->launches = 0;
   const size_t bytes = hm::upow(q, n) * sizeof(double2);
-  // split k so that about two CTAs per SM run, each over at least 256 values of k
+  // split k so that about two CTAs per SM run, each over at least 64 values of k (n = 18,
+  // NA = 7: 32 CTAs of 256 values took 95 us)
   const uint64_t tiles = ((dimA + hm::RT - 1) / hm::RT) * ((dimA + hm::RT - 1) / hm::RT);
   uint64_t nsplit = std::max<uint64_t>(1, (2 * (uint64_t)c->num_sms + tiles - 1) / tiles);
-  nsplit = std::min<uint64_t>(nsplit, std::max<uint64_t>(1, dimB / 256));
+  nsplit = std::min<uint64_t>(nsplit, std::max<uint64_t>(1, dimB / 64));
   nsplit = std::min<uint64_t>(nsplit, 1024);
   const uint64_t kps = ((dimB + nsplit - 1) / nsplit + hm::RK - 1) / hm::RK * hm::RK;
   nsplit = (dimB + kps - 1) / kps;
