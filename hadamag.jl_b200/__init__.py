@@ -371,7 +371,11 @@ def apply_2gate(sv, gate, s1, s2, device=0):
 def apply_brick_wall(sv, depth, gates, device=0):
     """Brick-wall circuit with the given gates (one per pair of brick_wall_pairs), in
     place, on the GPU (hm_brick_wall)."""
-    sv.data[:] = default_context(device).brick_wall(sv.data, sv.q, depth, list(gates))
+    ctx, v = default_context(device), sv.data
+    if v.dtype == np.complex128 and v.flags.c_contiguous and v.flags.writeable:
+        ctx.brick_wall_inplace(v, sv.q, depth, list(gates))
+    else:
+        v[:] = ctx.brick_wall(v, sv.q, depth, list(gates))
     return sv
 
 

@@ -319,7 +319,10 @@ class Context:
         if r.ndim != 2 or r.shape[0] != r.shape[1]:
             raise ArgumentError("DensityMatrix must be square")
         N = _log3_exact(r.shape[0])
-        col = np.ascontiguousarray(r.T)  # row-major bytes of r.T = column-major r
+        # The entry point takes column-major rho.  Row-major bytes are rho^T, and the sum of
+        # |tr(A_u rho^T)| = |tr(A_u^T rho)| over all phase points is the same one (transposing
+        # permutes the phase-point operators), so a row-major matrix goes as it is.
+        col = r if r.flags.c_contiguous else np.ascontiguousarray(r.T)
         v = ctypes.c_double()
         self._check(self.lib.hm_mana_mixed(self.handle, col.view(np.float64).ctypes.data_as(_dp), N,
                                            ctypes.byref(v)), "hm_mana_mixed")
@@ -363,8 +366,12 @@ class Context:
         return a
 
     def brick_wall(self, psi, q, depth, gates):
-        """Brick-wall circuit with one gate per site pair, in layer order."""
-        a = np.array(psi, dtype=np.complex128, copy=True)
+        """Brick-wall circuit with one gate per site pair, in layer order; returns the new
+        amplitudes."""
+        return self.brick_wall_inplace(np.array(psi, dtype=np.complex128, copy=True), q, depth, gates)
+
+    def brick_wall_inplace(self, a, q, depth, gates):
+        """As brick_wall, on the contiguous complex128 array `a` itself (unchanged on error)."""
         n = _logq_exact(a.size, q)
         gs = (np.ascontiguousarray(np.concatenate([_gate_colmajor(g, q) for g in gates])) if len(gates)
               else np.zeros(1, dtype=np.complex128))
