@@ -48,6 +48,40 @@ __device__ __forceinline__ void reg_wht(V (&v)[R]) {
   }
 }
 
+// One butterfly of registers i and i | 1 << S.
+template <int S, typename V>
+__device__ __forceinline__ void bfly(V (&v)[32], int i) {
+  const int k = i | (1 << S);
+  const V a = v[i], b = v[k];
+  v[i] = v_add(a, b);
+  v[k] = v_sub(a, b);
+}
+// The 32-register transforms run as 4 x 8: index bits 0, 1 inside each block of four
+// registers (as soon as the block has arrived), then bits 2 .. 4 inside each of the four
+// classes i mod 4 (each leaves as soon as it is done), so that the loads and stores of one
+// part overlap the arithmetic of another.
+template <int LO, int HI, typename V>
+__device__ __forceinline__ void wht_block(V (&v)[32], int b) {
+#pragma unroll
+  for (int i = 4 * b; i < 4 * b + 4; ++i)
+    if (LO <= 0 && HI > 0 && !(i & 1)) bfly<0>(v, i);
+#pragma unroll
+  for (int i = 4 * b; i < 4 * b + 4; ++i)
+    if (LO <= 1 && HI > 1 && !(i & 2)) bfly<1>(v, i);
+}
+template <int LO, int HI, typename V>
+__device__ __forceinline__ void wht_class(V (&v)[32], int c) {
+#pragma unroll
+  for (int i = c; i < 32; i += 4)
+    if (LO <= 2 && HI > 2 && !(i & 4)) bfly<2>(v, i);
+#pragma unroll
+  for (int i = c; i < 32; i += 4)
+    if (LO <= 3 && HI > 3 && !(i & 8)) bfly<3>(v, i);
+#pragma unroll
+  for (int i = c; i < 32; i += 4)
+    if (LO <= 4 && HI > 4 && !(i & 16)) bfly<4>(v, i);
+}
+
 // layout A -> layout B through a warp-private buffer of 32R elements
 template <int R, typename V>
 __device__ __forceinline__ void transpose_ab(V (&v)[R], V *sm, int lane) {
@@ -63,6 +97,34 @@ __device__ __forceinline__ void transpose_ab(V (&v)[R], V *sm, int lane) {
   for (int i = 0; i < R; ++i) {
     const int e = lane * R + i;
     v[i] = sm[e ^ ((e >> LOGR) & SW)];
+  }
+  __syncwarp();
+}
+
+// The register butterflies of layout A over bits 2 .. 4 (bits 0, 1 done by block before), the
+// exchange, and those of layout B over bits LO .. 1: the classes store as they finish, the
+// blocks start as they arrive.  What is left of layout B is bits 2 .. 4, by class.
+template <int LO, typename V>
+__device__ __forceinline__ void wht_exchange(V (&v)[32], V *sm, int lane) {
+  constexpr int SW = 128 / (int)sizeof(V) - 1;
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    wht_class<2, 5>(v, c);
+#pragma unroll
+    for (int i = c; i < 32; i += 4) {
+      const int e = i * 32 + lane;
+      sm[e ^ ((e >> 5) & SW)] = v[i];
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int b = 0; b < 8; ++b) {
+#pragma unroll
+    for (int i = 4 * b; i < 4 * b + 4; ++i) {
+      const int e = lane * 32 + i;
+      v[i] = sm[e ^ ((e >> 5) & SW)];
+    }
+    wht_block<LO, 2>(v, b);
   }
   __syncwarp();
 }
@@ -247,6 +309,44 @@ __device__ __forceinline__ void lane_moments(const V (&v)[R], double *s, const Q
   }
 }
 
+// Sums of one quad of values before its last two butterfly levels.  With c_d = sum_e u_e
+// u_(e^d) the four outputs satisfy sum F^2 = 4 c_0 and sum F^4 = 4 (c_0^2 + c_1^2 + c_2^2 +
+// c_3^2) (F_k^2 = sum_d (-1)^(k.d) c_d, Parseval over k): 15 operations for the four values
+// instead of 8 for the two levels and 12 for the powers.
+struct QuadSums {
+  double a2[2] = {0.0, 0.0}, m0[2] = {0.0, 0.0}, h1 = 0.0, h2 = 0.0, h3 = 0.0;
+  __device__ __forceinline__ void add(int t, double u0, double u1, double u2, double u3) {
+    const double c0 = fma(u0, u0, fma(u1, u1, fma(u2, u2, u3 * u3)));
+    const double c1 = fma(u0, u1, u2 * u3), c2 = fma(u0, u2, u1 * u3), c3 = fma(u0, u3, u1 * u2);
+    a2[t] += c0;
+    m0[t] = fma(c0, c0, m0[t]);
+    h1 = fma(c1, c1, h1);
+    h2 = fma(c2, c2, h2);
+    h3 = fma(c3, c3, h3);
+  }
+  __device__ __forceinline__ void get(double *s) const {
+    s[0] = 4.0 * (a2[0] + a2[1]);
+    s[1] = 4.0 * ((m0[0] + m0[1]) + 4.0 * ((h1 + h2) + h3));
+  }
+};
+
+// q = 2 sums of 32 complex registers whose register bits LO .. 4 are still to transform (bits
+// below 2 done): bit 2 if it is one of them, then quads over bits 3 and 4
+template <int LO, typename V>
+__device__ __forceinline__ void quad_moments(V (&v)[32], double *s) {
+  QuadSums q;
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    if constexpr (LO <= 2) wht_class<2, 3>(v, c);
+#pragma unroll
+    for (int i = c; i < 8; i += 4) {
+      q.add(0, v[i].x, v[i + 8].x, v[i + 16].x, v[i + 24].x);
+      q.add(1, v[i].y, v[i + 8].y, v[i + 16].y, v[i + 24].y);
+    }
+  }
+  q.get(s);
+}
+
 // scale of sum (F^2)^q for one X-string: F = 2 W (x != 0) or W (x = 0)
 template <int QS>
 __device__ __forceinline__ double q_scale(int t, bool xzero, const QParams &qp) {
@@ -423,23 +523,29 @@ __device__ __forceinline__ void p1_unit_tma(const V *__restrict__ psi, const XIn
   constexpr int LOGR = ilog2c(R);
   V v[R];
   p1_build<R, false>(v, psi, xi, rho, sm, lane);  // registers only (no shared memory)
+#ifdef HM_TMEM_EXCHANGE
   reg_wht<R, 0, LOGR>(v);
   ready();  // the shared buffer is free from here on
-#ifdef HM_TMEM_EXCHANGE
-  if constexpr (TM) {
-    static_assert(R == 32, "the TMEM exchanges are generated for 32 values per lane");
-    tmem_row(v, ta);
-  } else {
-    transpose_ab<R>(v, sm, lane);
-  }
-#else
-  (void)ta;
-  transpose_ab<R>(v, sm, lane);
-#endif
+  static_assert(TM && R == 32, "the TMEM exchanges are generated for 32 values per lane");
+  tmem_row(v, ta);
   reg_wht<R, 0, 5>(v);
-  // register i of lane l holds element k = R l + i, kept at position p = 32 i + l
 #pragma unroll
   for (int i = 0; i < R; ++i) sm[i * 32 + lane] = v[i];
+#else
+  (void)ta;
+  static_assert(R == 32 && LOGR == 5, "32 values per lane");
+#pragma unroll
+  for (int b = 0; b < 8; ++b) wht_block<0, 2>(v, b);
+  ready();  // the shared buffer is free from here on
+  wht_exchange<0>(v, sm, lane);
+  // register i of lane l holds element k = R l + i, kept at position p = 32 i + l
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    wht_class<2, 5>(v, c);
+#pragma unroll
+    for (int i = c; i < 32; i += 4) sm[i * 32 + lane] = v[i];
+  }
+#endif
   fence_proxy_async_smem();
   __syncwarp();
   pre();
@@ -474,10 +580,17 @@ __device__ __forceinline__ void p2_unit(const V *__restrict__ tile_ptr, V *sm, i
     reg_wht<R, 0, 5 - LOGC>(v);
 #endif
   } else {
-    reg_wht<R, 0, LOGR>(v);
+    static_assert(R == 32, "32 values per lane");
+#pragma unroll
+    for (int b = 0; b < 8; ++b) wht_block<0, 2>(v, b);
     ready();
-    transpose_ab<R>(v, sm, lane);
-    reg_wht<R, LOGC, 5>(v);
+    wht_exchange<(LOGC < 2 ? LOGC : 2)>(v, sm, lane);
+    if constexpr (QS == QS_Q2 && LOGC <= 3) {
+      quad_moments<LOGC>(v, s);
+      return;
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) wht_class<(LOGC > 2 ? LOGC : 2), 5>(v, c);
   }
   lane_moments<R, QS>(v, s, qp, sm, lane);
 }

@@ -25,9 +25,10 @@ namespace hm {
 //         n = 21: X = 4 (4.65; 2: 4.90)
 // Against the rows and tiles of k_sre_stage, which ran every size before: FP64 0.116, 0.206,
 // 0.430, 0.852, 1.815, 3.79, 10.33 for n = 15 .. 21, FP32 0.067, 0.115, 0.221, 0.446, 0.967,
-// 2.70, 10.02.  FP64 at n = 20 stays with k_sre_stage (X = 10: 3.79; 3.87 here at X = 7):
-// both are bound by the ring's traffic there, and its tensor stores need no group of four.
-// So does FP64 at n = 19 for q = 2 and 3 together (X = 16: 1.88; 1.91 here).
+// 2.70, 10.02.  FP64 at n = 20 stays with k_sre_stage (X = 10: 3.74, 3.83 before its q = 2
+// moments by quads; 3.87 here at X = 7): both are bound by the ring's traffic there, and its
+// tensor stores need no group of four.  So does FP64 at n = 19 for q = 2 and 3 together
+// (X = 16: 1.89; 1.91 here).
 // hm_autotune measures and records a batch for the machine at hand; setting
 // HM_PARAM_BATCH, _UNITS or _RING switches to the generic rule.
 inline int measured_x(bool fp64, int n) {

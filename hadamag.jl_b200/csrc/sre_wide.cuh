@@ -25,40 +25,6 @@
 
 namespace hm {
 
-// One butterfly of registers i and i | 1 << S.
-template <int S, typename V>
-__device__ __forceinline__ void bfly(V (&v)[32], int i) {
-  const int k = i | (1 << S);
-  const V a = v[i], b = v[k];
-  v[i] = v_add(a, b);
-  v[k] = v_sub(a, b);
-}
-// The 32-register transforms run as 4 x 8: index bits 0, 1 inside each block of four
-// registers (as soon as the block has arrived), then bits 2 .. 4 inside each of the four
-// classes i mod 4 (each leaves as soon as it is done), so that the loads and stores of one
-// part overlap the arithmetic of another.
-template <int LO, int HI, typename V>
-__device__ __forceinline__ void wht_block(V (&v)[32], int b) {
-#pragma unroll
-  for (int i = 4 * b; i < 4 * b + 4; ++i)
-    if (LO <= 0 && HI > 0 && !(i & 1)) bfly<0>(v, i);
-#pragma unroll
-  for (int i = 4 * b; i < 4 * b + 4; ++i)
-    if (LO <= 1 && HI > 1 && !(i & 2)) bfly<1>(v, i);
-}
-template <int LO, int HI, typename V>
-__device__ __forceinline__ void wht_class(V (&v)[32], int c) {
-#pragma unroll
-  for (int i = c; i < 32; i += 4)
-    if (LO <= 2 && HI > 2 && !(i & 4)) bfly<2>(v, i);
-#pragma unroll
-  for (int i = c; i < 32; i += 4)
-    if (LO <= 3 && HI > 3 && !(i & 8)) bfly<3>(v, i);
-#pragma unroll
-  for (int i = c; i < 32; i += 4)
-    if (LO <= 4 && HI > 4 && !(i & 16)) bfly<4>(v, i);
-}
-
 // threads of one group meet (id 0 .. 15; the group's warps are whole warps)
 template <int NT>
 __device__ __forceinline__ void group_sync(int id) {
@@ -229,26 +195,14 @@ __device__ __noinline__ void wide_moments_gen(const T *sm, int lane, double *s, 
 
 // Butterflies over the LV low bits of the register index (and, with PAIR, over the bit inside
 // a pair), then the per-lane sums of F^2 and (F^2)^q.
-// q = 2 alone: the last two bits are not transformed.  For four values u_e before them,
-// with c_d = sum_e u_e u_(e^d), the four outputs satisfy sum F^2 = 4 c_0 and
-// sum F^4 = 4 (c_0^2 + c_1^2 + c_2^2 + c_3^2) (F_k^2 = sum_d (-1)^(k.d) c_d, Parseval over k):
-// 15 operations for the four values instead of 8 for the two bits and 12 for the powers.
+// q = 2 alone: the last two bits are not transformed (QuadSums).
 template <int QS, int LV, bool PAIR, typename T, typename V>
 __device__ __forceinline__ void wide_moments(V (&v)[32], double *s, const QParams &qp, T *sm, int lane) {
   if constexpr (QS == QS_Q2) {
     constexpr int TOP = PAIR ? LV - 1 : LV - 2;  // transformed explicitly: index bits 0 .. TOP-1
 #pragma unroll
     for (int b = 0; b < 8; ++b) wht_block<0, TOP>(v, b);
-    double a2[2] = {0.0, 0.0}, m0[2] = {0.0, 0.0}, h1 = 0.0, h2 = 0.0, h3 = 0.0;
-    auto quad = [&](int t, double u0, double u1, double u2, double u3) {
-      const double c0 = fma(u0, u0, fma(u1, u1, fma(u2, u2, u3 * u3)));
-      const double c1 = fma(u0, u1, u2 * u3), c2 = fma(u0, u2, u1 * u3), c3 = fma(u0, u3, u1 * u2);
-      a2[t] += c0;
-      m0[t] = fma(c0, c0, m0[t]);
-      h1 = fma(c1, c1, h1);
-      h2 = fma(c2, c2, h2);
-      h3 = fma(c3, c3, h3);
-    };
+    QuadSums quad;
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       wht_class<0, TOP>(v, c);
@@ -257,17 +211,16 @@ __device__ __forceinline__ void wide_moments(V (&v)[32], double *s, const QParam
       if constexpr (PAIR) {
         if ((i >> TOP) & 1) continue;
         const int k = i | (1 << TOP);
-        quad(i & 1, v[i].x, v[i].y, v[k].x, v[k].y);
+        quad.add(i & 1, v[i].x, v[i].y, v[k].x, v[k].y);
       } else {
         if ((i >> TOP) & 3) continue;
         const int k = i | (1 << TOP), m = i | (2 << TOP);
-        quad(0, v[i].x, v[k].x, v[m].x, v[m | k].x);
-        quad(1, v[i].y, v[k].y, v[m].y, v[m | k].y);
+        quad.add(0, v[i].x, v[k].x, v[m].x, v[m | k].x);
+        quad.add(1, v[i].y, v[k].y, v[m].y, v[m | k].y);
       }
     }
     }
-    s[0] = 4.0 * (a2[0] + a2[1]);
-    s[1] = 4.0 * ((m0[0] + m0[1]) + 4.0 * ((h1 + h2) + h3));
+    quad.get(s);
   } else {
     reg_wht<32, 0, LV>(v);
     if constexpr (PAIR) {
