@@ -18,7 +18,7 @@ namespace hm {
 // X = 37 m at n = 17) within a ring of about 120 MiB, timed on B200 (us per X-string):
 //   FP64  n = 15: X = 148 (0.107; 74: 0.120)    n = 16: X = 111 (0.191; 74: 0.195, 37: 0.22)
 //         n = 17: X = 55 (0.377; 37: 0.387)     n = 18: X = 27 (0.784; 18: 0.785, 37: 0.796)
-//         n = 19: X = 9 (1.735; 14: 1.759, 4: 1.83)  n = 21: X = 2 (9.40; 3: 9.68)
+//         n = 19: X = 9 (1.735; 14: 1.759, 4: 1.83)  n = 21: X = 4 (9.10; 3: 9.29, 2: 9.87)
 //   FP32  n = 15: X = 296 (0.062; 256: 0.070)  n = 16: X = 148 (0.106; 74: 0.124)
 //         n = 17: X = 110 (0.197; 74: 0.204)    n = 18: X = 55 (0.403; 37: 0.413)
 //         n = 19: X = 18 (0.861; 28: 0.878)     n = 20: X = 9 (1.97; 7: 2.02)
@@ -32,7 +32,7 @@ namespace hm {
 // hm_autotune measures and records a batch for the machine at hand; setting
 // HM_PARAM_BATCH, _UNITS or _RING switches to the generic rule.
 inline int measured_x(bool fp64, int n) {
-  static const int f64[7] = {148, 111, 55, 27, 9, 10, 2}, f32[7] = {296, 148, 110, 55, 18, 9, 4};
+  static const int f64[7] = {148, 111, 55, 27, 9, 10, 4}, f32[7] = {296, 148, 110, 55, 18, 9, 4};
   return (n >= 15 && n <= 21) ? (fp64 ? f64 : f32)[n - 15] : 0;
 }
 
@@ -248,10 +248,11 @@ static int launch_stages(hm_ctx *c, const SreArgs &a0, int *nwarps_out) {
 
 // Warps per pass-1 group of the two-pass sweep at n qubits: two (rows of 2048 complex
 // values), more from the size on where pass 2 would otherwise hold more than one row bit on
-// lane bits and read less than 128 bytes per row and unit, whole lines that it can discard
-// (FP32 at n = 19: 0.861 us per X-string with four, 0.966 with two).
+// lane bits and read less than 128 bytes per row and unit (FP32 at n = 19: 0.861 us per
+// X-string with four, 0.966 with two).  Past n = 20 the units of a warp are paired to whole
+// lines anyway; FP64 at n = 21: 9.10 with four and pairs, 9.40 with eight.
 template <typename T> constexpr int wide_group(int n) {
-  return n <= (sizeof(T) == 8 ? 19 : 18) ? 2 : n <= 20 ? 4 : 8;
+  return n <= (sizeof(T) == 8 ? 19 : 18) ? 2 : n <= (sizeof(T) == 8 ? 21 : 20) ? 4 : 8;
 }
 
 // Two-pass sweep (see k_sre_wide_stage): ring of two batches, stages chained and replayed

@@ -384,11 +384,15 @@ __global__ void __launch_bounds__(32 * WideCta<G>::WARPS, (sizeof(T) == 8 ? 8 : 
   T *ring = reinterpret_cast<T *>(a.ring);
   const long long per = (long long)a.X * NROW;    // items (row or G column blocks) per pass
   const long long n1 = t < a.nbatch ? per : 0;    // pass 1 of batch t
-  const long long n2 = t >= 1 ? per : 0;          // pass 2 of batch t - 1
+  constexpr uint32_t CHUNK = (2048u >> HI) * sizeof(T);    // bytes of a unit in each row
+  constexpr uint32_t UPI = CHUNK < 128 ? 128 / CHUNK : 1;  // units per item: whole L2 lines
+  const long long n2 = t >= 1 ? per / UPI : 0;             // pass 2 of batch t - 1
   const long long gid = (long long)blockIdx.x * NG + grp, ngrp = (long long)gridDim.x * NG;
   dd acc[NQ + 1];
 #pragma unroll
   for (int q = 0; q <= NQ; ++q) acc[q] = dd{0.0, 0.0};
+  // One pass-1 item first (its gathers and butterflies overlap the previous stage's tail), then
+  // the pass-2 items (the previous stage's rows are still in L2), then the rest of pass 1.
   const long long nfirst = n1 < ngrp ? n1 : ngrp;
   for (long long u = gid; u < n1 + n2; u += ngrp) {
     const bool p2 = u >= nfirst && u < nfirst + n2;
@@ -424,47 +428,48 @@ __global__ void __launch_bounds__(32 * WideCta<G>::WARPS, (sizeof(T) == 8 ? 8 : 
       }
     } else {
       wait_prior_grid();  // the previous stage's rows
-      const uint32_t unit = sub * G + w;  // block of 2^(11-HI) columns
-      const T *col = inter + ((size_t)unit << (11 - HI));
-      double s[NQ + 1];
-      if constexpr (HI <= 5) {
-        // register i: row i mod 2^HI, column block i >> HI of 64 columns (a pair per lane)
+#pragma unroll 1
+      for (uint32_t h = 0; h < UPI; ++h) {
+        const uint32_t unit = (sub * G + w) * UPI + h;  // block of 2^(11-HI) columns
+        const T *col = inter + ((size_t)unit << (11 - HI));
+        double s[NQ + 1];
+        if constexpr (HI <= 5) {
+          // register i: row i mod 2^HI, column block i >> HI of 64 columns (a pair per lane)
 #pragma unroll
-        for (int i = 0; i < 32; ++i)
-          v[i] = __ldcg(reinterpret_cast<const V *>(col + (size_t)(i & (NROW - 1)) * ROW + 64 * (i >> HI)) + lane);
-      } else {
-        // lane: column in its low 11 - HI bits, the row's low HI - 6 bits above them;
-        // register pair i: rows with bits HI-6 = (x, y) and i above
-        constexpr int CB = 11 - HI, LB = HI - 6;
-        const T *p = col + (lane & ((1 << CB) - 1)) + (size_t)(lane >> CB) * ROW;
+          for (int i = 0; i < 32; ++i)
+            v[i] = __ldcg(reinterpret_cast<const V *>(col + (size_t)(i & (NROW - 1)) * ROW + 64 * (i >> HI)) + lane);
+        } else {
+          // lane: column in its low 11 - HI bits, the row's low HI - 6 bits above them;
+          // register pair i: rows with bits HI-6 = (x, y) and i above
+          constexpr int CB = 11 - HI, LB = HI - 6;
+          const T *p = col + (lane & ((1 << CB) - 1)) + (size_t)(lane >> CB) * ROW;
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          v[i].x = __ldcg(p + (size_t)((2 * i) << LB) * ROW);
-          v[i].y = __ldcg(p + (size_t)((2 * i + 1) << LB) * ROW);
+          for (int i = 0; i < 32; ++i) {
+            v[i].x = __ldcg(p + (size_t)((2 * i) << LB) * ROW);
+            v[i].y = __ldcg(p + (size_t)((2 * i + 1) << LB) * ROW);
+          }
+#pragma unroll
+          for (int m = 1 << CB; m < 32; m <<= 1) lane_wht(v, lane, m);
         }
+        if constexpr (QS == QS_GEN) group_sync<32 * G>(1 + grp);  // the moments stage in the buffer
+        wide_moments<QS, (HI <= 5 ? HI : 5), (HI > 5)>(v, s, a.qp, buf + 2048 * w, lane);
+        s[0] = x == 0 ? s[0] : 4.0 * s[0];
 #pragma unroll
-        for (int m = 1 << CB; m < 32; m <<= 1) lane_wht(v, lane, m);
+        for (int q = 0; q < NQ; ++q) s[1 + q] *= q_scale<QS>(q, x == 0, a.qp);
+#pragma unroll
+        for (int q = 0; q <= NQ; ++q) dd_add(acc[q], s[q]);
       }
-      if constexpr (QS == QS_GEN) group_sync<32 * G>(1 + grp);  // the moments stage in the buffer
-      wide_moments<QS, (HI <= 5 ? HI : 5), (HI > 5)>(v, s, a.qp, buf + 2048 * w, lane);
       // The columns are dead once read (their slot is rewritten two stages later, after
       // griddepcontrol.wait on the launch in between): drop their L2 lines without writing
-      // them back.  A unit owns whole 128-byte lines when its row chunk is at least that.
-      constexpr uint32_t CHUNK = (2048u >> HI) * sizeof(T);
-      if constexpr (CHUNK >= 128) {
-        constexpr uint32_t LPR = CHUNK / 128;  // lines per row
-        __syncwarp();                          // every lane's reads come before
+      // them back.
+      constexpr uint32_t LPR = CHUNK * UPI / 128;  // lines per row
+      const T *line = inter + ((size_t)((sub * G + w) * UPI) << (11 - HI));
+      __syncwarp();  // every lane's reads come before
 #pragma unroll
-        for (uint32_t ln = lane; ln < NROW * LPR; ln += 32)
-          asm volatile("discard.global.L2 [%0], 128;" ::"l"(reinterpret_cast<const char *>(
-                           col + (size_t)(ln / LPR) * ROW) + (ln % LPR) * 128)
-                       : "memory");
-      }
-      s[0] = x == 0 ? s[0] : 4.0 * s[0];
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) s[1 + q] *= q_scale<QS>(q, x == 0, a.qp);
-#pragma unroll
-      for (int q = 0; q <= NQ; ++q) dd_add(acc[q], s[q]);
+      for (uint32_t ln = lane; ln < NROW * LPR; ln += 32)
+        asm volatile("discard.global.L2 [%0], 128;" ::"l"(reinterpret_cast<const char *>(
+                         line + (size_t)(ln / LPR) * ROW) + (ln % LPR) * 128)
+                     : "memory");
     }
   }
   if (n2 > 0) {
