@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(128) k_adj_fused(AdjArgs a) {
     transpose_ab<R>(v, sm, lane);
     reg_wht<R, 0, (NB < 5 ? NB : 5)>(v);
     const int qi = (int)a.q;
-    mloc = adj_pointwise<0>(v, qi, xz ? a.cq_0 : a.cq_x, sm, lane) * (xz ? 1.0 : pow_q_dev(4.0, a.q));
+    mloc = adj_pointwise<0>(v, qi, xz ? a.cq_0 : a.cq_x, sm, lane) * (xz ? 1.0 : scalbn(1.0, 2 * (int)a.q));
     reg_wht<R, 0, (NB < 5 ? NB : 5)>(v);
     transpose_ba(v, sm, lane);
     if constexpr (NB > 5) reg_wht<R, 0, NB - 5>(v);
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(128) k_adj_p2(AdjArgs a) {
       transpose_ab<R>(v, sm, lane);
       reg_wht<R, LOGC, 5>(v);
     }
-    mloc = adj_pointwise<0>(v, (int)a.q, xz ? a.cq_0 : a.cq_x, sm, lane) * (xz ? 1.0 : pow_q_dev(4.0, a.q));
+    mloc = adj_pointwise<0>(v, (int)a.q, xz ? a.cq_0 : a.cq_x, sm, lane) * (xz ? 1.0 : scalbn(1.0, 2 * (int)a.q));
     if constexpr (LOGC >= 5) {
       reg_wht<R, LOGC - 5, 5>(v);
     } else {

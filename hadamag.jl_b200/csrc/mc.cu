@@ -48,7 +48,7 @@ struct McArgs {
 // q = 2 or generic through QS_GEN
 template <int QS>
 __device__ __forceinline__ double moment_scale(const QParams &qp) {
-  return QS == QS_Q2 ? 16.0 : pow_q_dev(4.0, qp.q[0]);
+  return QS == QS_Q2 ? 16.0 : qp.scale[0];
 }
 
 // n >= 16, pass 1: warp units (chain, row)
@@ -97,9 +97,7 @@ __global__ void __launch_bounds__(128) k_mc_p2(McArgs a) {
   const uint64_t tile = (uint64_t)(u % a.U);
   if (a.ch[c].prop == 0) return;
   double s[5];
-  QParams qp = a.qp;
-  qp.nq = 1;
-  p2_unit<R, HI, QS>(a.inter + (size_t)c * ((size_t)1 << (a.n - 1)) + (tile << PB), sm, lane, s, qp);
+  p2_unit<R, HI, QS>(a.inter + (size_t)c * ((size_t)1 << (a.n - 1)) + (tile << PB), sm, lane, s, a.qp);
   const double p2 = warp_sum(s[0]) * 4.0, m = warp_sum(s[1]) * moment_scale<QS>(a.qp);
   if (lane == 0) {
     a.part[2 * u] = p2;
@@ -238,8 +236,6 @@ __global__ void __launch_bounds__(32) k_mc_chain_warp(McArgs a) {
   const int c = blockIdx.x, lane = threadIdx.x;
   McChain ch;
   ch.start(a, c);
-  QParams qp = a.qp;
-  qp.nq = 1;
   for (int t = 0; t < a.nsamples; ++t) {
     ch.fetch(a, t);
     double p2 = 0.0, m = 0.0;
@@ -260,7 +256,7 @@ __global__ void __launch_bounds__(32) k_mc_chain_warp(McArgs a) {
       transpose_ab<R>(v, sm, lane);
       reg_wht<R, 0, (NB < 5 ? NB : 5)>(v);
       double s[5];
-      lane_moments<R, QS>(v, s, qp, sm, lane);
+      lane_moments<R, QS>(v, s, a.qp, sm, lane);
       p2 = warp_sum(s[0]) * 4.0;
       m = warp_sum(s[1]) * moment_scale<QS>(a.qp);
     }
@@ -319,8 +315,6 @@ __global__ void __launch_bounds__(32 * ((1 << L) / CS), 8 / ((1 << L) / CS)) k_m
   for (int k = 0; k < CS; ++k) peer[k] = chain_addr<CS>((uint32_t)__cvta_generic_to_shared(buf), k);
   McChain ch;
   ch.start(a, c);
-  QParams qp = a.qp;
-  qp.nq = 1;
   if constexpr (CS > 1) chain_sync<CS>();  // every CTA of the cluster runs before remote stores
   for (int t = 0; t < a.nsamples; ++t) {
     ch.fetch(a, t);
@@ -355,7 +349,7 @@ __global__ void __launch_bounds__(32 * ((1 << L) / CS), 8 / ((1 << L) / CS)) k_m
       double s[5];
       if constexpr (L <= 2) {
         if constexpr (L == 2) lane_wht(v, lane, 1);
-        wide_moments<QS, 5, true>(v, s, qp, slice, lane);
+        wide_moments<QS, 5, true>(v, s, a.qp, slice, lane);
       } else {
 #pragma unroll
         for (int b = 0; b < 8; ++b) wht_block<0, 2>(v, b);
@@ -368,7 +362,7 @@ __global__ void __launch_bounds__(32 * ((1 << L) / CS), 8 / ((1 << L) / CS)) k_m
           v[i].y = p - q;
         }
         transpose_ab<32>(v, reinterpret_cast<double2 *>(slice), lane);
-        wide_moments<QS, L - 1, false>(v, s, qp, slice, lane);
+        wide_moments<QS, L - 1, false>(v, s, a.qp, slice, lane);
       }
       p2 = warp_sum(s[0]) * 4.0;
       m = warp_sum(s[1]) * moment_scale<QS>(a.qp);
@@ -601,8 +595,7 @@ int run_mc(hm_ctx *c, const double2 *psi, int n, double q, int nbeta_grid, int c
   a.nsamples = nsamples;
   a.pd = pd_dev;
   a.rs = rs_dev;
-  a.qp.q[0] = q;
-  a.qp.nq = 1;
+  set_qparams(a.qp, &q, 1);
   const bool q2 = (q == 2.0);
   a.p2_0 = p2_0;
   a.m0 = m0;

@@ -159,8 +159,7 @@ extern "C" int hm_sre_noalloc(const double *psi, int n, const double *qs, int nq
     for (int i = 0; i < nq; ++i) idx[i] = qs[i] == 2.0 ? 1 : 2;
   } else {
     kind = hm::QS_GEN;
-    qp.nq = nq;
-    for (int i = 0; i < 4; ++i) qp.q[i] = i < nq ? qs[i] : 2.0;
+    hm::set_qparams(qp, qs, nq);
     for (int i = 0; i < nq; ++i) idx[i] = 1 + i;
   }
   const int nsum = 1 + (kind == hm::QS_Q2 ? 1 : (kind == hm::QS_Q23 ? 2 : 4));

@@ -224,41 +224,106 @@ template <int QS> struct QSet {
 
 struct QParams {
   double q[4];
+  double scale[4];  // 4^q
   int nq;
+  int direct;  // one q, an integer or a half-integer (half_integer_q)
 };
 
-__device__ __forceinline__ double pow_q_dev(double y, double q) {
-  // integer q in [1,16]: repeated squaring; otherwise pow
-  if (q == floor(q) && q >= 1.0 && q <= 16.0) {
-    int e = (int)q;
-    double r = 1.0, b = y;
-    while (e) {
-      if (e & 1) r *= b;
-      b *= b;
-      e >>= 1;
-    }
-    return r;
+// (F^2)^q with 2q an integer is F^2 to an integer power, times |F| if 2q is odd
+__host__ __device__ inline bool half_integer_q(double q) { return 2.0 * q == floor(2.0 * q) && q >= 1.0 && q <= 16.0; }
+
+inline void set_qparams(QParams &qp, const double *q, int nq) {
+  qp.nq = nq;
+  qp.direct = nq == 1 && half_integer_q(q[0]);
+  for (int i = 0; i < 4; ++i) {
+    qp.q[i] = i < nq ? q[i] : 2.0;
+    qp.scale[i] = pow(4.0, qp.q[i]);
   }
-  return pow(y, q);
 }
 
-// Per-lane sums of F^2 and of (F^2)^q over the R complex registers (2R values of F/2
-// for x != 0; the caller applies the 4 / 4^q scale), plain FP64 sums in a fixed order.
-// Generic Renyi indices: the F values go through the warp's shared buffer so that the
-// pow() evaluations run in a rolled loop instead of an unrolled register sweep.
+// y^q and |f| y^(q - 1/2) for y = f^2, half_integer_q(q), N values side by side: the bits of
+// the exponent from the second one down, square and multiply.
+template <int N>
+__device__ __forceinline__ void pow_half(const double (&f)[N], const double (&y)[N], double q, double (&r)[N]) {
+  const int e2 = (int)(2.0 * q), e = e2 >> 1;
+#pragma unroll
+  for (int t = 0; t < N; ++t) r[t] = y[t];
+#pragma unroll 1
+  for (int b = 30 - __clz(e); b >= 0; --b) {
+#pragma unroll
+    for (int t = 0; t < N; ++t) r[t] *= r[t];
+    if ((e >> b) & 1) {
+#pragma unroll
+      for (int t = 0; t < N; ++t) r[t] *= y[t];
+    }
+  }
+  if (e2 & 1) {
+#pragma unroll
+    for (int t = 0; t < N; ++t) r[t] *= fabs(f[t]);
+  }
+}
+
+// Generic Renyi indices, per-lane sums of F^2 and (F^2)^q of the R complex registers.
+//   one half-integer q (qp.direct): from the registers, 16 values at a time (FP32: 8, for
+//     its 128 registers), so that the powers are independent chains over the FP64 latency; the
+//     exponent is uniform over the grid.  A step of the loop over its bits is one product per
+//     value.  FP64 on B200, all 2^n X-strings: n = 13 q = 4 318 -> 155 us (staged, four chains),
+//     q = 2.5 1.50 ms -> 155 us (pow); n = 11 q = 4 52 -> 33 us; n = 20 q = 4 7.2 -> 5.0 us each.
+//     Error of the sums against extended precision, n = 6 .. 11: 7e-16 at q = 2.5 (pow 13e-16).
+//     (A list of several q would keep all values and the sums in registers, which spill.)
 template <int R, typename V>
-__device__ __noinline__ void lane_moments_gen(const V *sm, int lane, double *s, const QParams &qp) {
+__device__ __forceinline__ void lane_moments_direct(const V (&v)[R], double *s, const QParams &qp) {
+  constexpr int N = sizeof(V) == 16 ? 16 : 8;
+  double a2 = 0.0, ag = 0.0;
+#pragma unroll
+  for (int c = 0; c < 2 * R / N; ++c) {
+    double f[N], y[N], r[N];
+#pragma unroll
+    for (int t = 0; t < N; ++t) {
+      f[t] = (double)(t & 1 ? v[(c * N + t) / 2].y : v[(c * N + t) / 2].x);
+      y[t] = f[t] * f[t];
+    }
+    pow_half(f, y, qp.q[0], r);
+#pragma unroll
+    for (int w = N / 2; w > 0; w >>= 1)
+#pragma unroll
+      for (int t = 0; t < w; ++t) {
+        y[t] += y[t + w];
+        r[t] += r[t + w];
+      }
+    a2 += y[0];
+    ag += r[0];
+  }
+  s[0] = a2;
+  s[1] = ag;
+#pragma unroll
+  for (int t = 1; t < 4; ++t) s[1 + t] = 0.0;
+}
+
+//   others: the F values go through the warp's own shared buffer (sm[lane + 32 t], NV of
+//     them), so that the pow() evaluations run in a rolled loop, four chains at a time.
+template <int NV, typename T>
+__device__ __noinline__ void lane_moments_gen(const T *sm, int lane, double *s, const QParams &qp) {
   double a2 = 0.0, ag[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll 1
-  for (int i = 0; i < R; ++i) {
-    const V f2 = sm[lane + 32 * i];
+  for (int t0 = 0; t0 < NV; t0 += 4) {
+    double f[4], y[4], r[4];
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const double f = c ? (double)f2.y : (double)f2.x;
-      const double y = f * f;
-      a2 += y;
+    for (int t = 0; t < 4; ++t) {
+      f[t] = (double)sm[lane + 32 * (t0 + t)];
+      y[t] = f[t] * f[t];
+    }
+    a2 += (y[0] + y[1]) + (y[2] + y[3]);
 #pragma unroll 1
-      for (int t = 0; t < qp.nq; ++t) ag[t] += pow_q_dev(y, qp.q[t]);
+    for (int k = 0; k < qp.nq; ++k) {
+      const double q = qp.q[k];
+      if (half_integer_q(q)) {
+        pow_half(f, y, q, r);
+      } else {
+#pragma unroll
+        for (int t = 0; t < 4; ++t) r[t] = pow(y[t], q);
+      }
+      ag[k] += (r[0] + r[1]) + (r[2] + r[3]);
     }
   }
   s[0] = a2;
@@ -266,6 +331,8 @@ __device__ __noinline__ void lane_moments_gen(const V *sm, int lane, double *s, 
   for (int t = 0; t < 4; ++t) s[1 + t] = ag[t];
 }
 
+// Per-lane sums of F^2 and of (F^2)^q over the R complex registers (2R values of F/2
+// for x != 0; the caller applies the 4 / 4^q scale), plain FP64 sums in a fixed order.
 // Both precisions take the powers and the sums in FP64: an FP32 value of F converts to
 // double exactly, so the FP32 path's only roundings are those of f and of the butterflies.
 // NA interleaved accumulators per sum (value j goes to accumulator j mod NA, combined
@@ -273,9 +340,17 @@ __device__ __noinline__ void lane_moments_gen(const V *sm, int lane, double *s, 
 template <int R, int QS, typename V>
 __device__ __forceinline__ void lane_moments(const V (&v)[R], double *s, const QParams &qp, V *sm, int lane) {
   if constexpr (QS == QS_GEN) {
+    if (qp.direct) {
+      lane_moments_direct(v, s, qp);
+      return;
+    }
+    auto *f = &sm->x;
 #pragma unroll
-    for (int i = 0; i < R; ++i) sm[lane + 32 * i] = v[i];
-    lane_moments_gen<R>(sm, lane, s, qp);
+    for (int i = 0; i < R; ++i) {
+      f[lane + 32 * (2 * i)] = v[i].x;
+      f[lane + 32 * (2 * i + 1)] = v[i].y;
+    }
+    lane_moments_gen<2 * R>(f, lane, s, qp);
     __syncwarp();
     return;
   } else {
@@ -353,7 +428,7 @@ __device__ __forceinline__ double q_scale(int t, bool xzero, const QParams &qp) 
   if (xzero) return 1.0;
   if constexpr (QS == QS_Q2) return 16.0;
   if constexpr (QS == QS_Q23) return t == 0 ? 16.0 : 64.0;
-  return pow_q_dev(4.0, qp.q[t]);
+  return qp.scale[t];
 }
 
 // ---------------------------------------------------------------------------------

@@ -126,12 +126,8 @@ static int choose_qs(const QReq &q, QParams &qp, int *idx) {
     for (int i = 0; i < q.nq; ++i) idx[i] = q.q[i] == 2.0 ? 1 : 2;
     return QS_Q23;
   }
-  qp.nq = q.nq;
-  for (int i = 0; i < q.nq; ++i) {
-    qp.q[i] = q.q[i];
-    idx[i] = 1 + i;
-  }
-  for (int i = q.nq; i < 4; ++i) qp.q[i] = 2.0;
+  set_qparams(qp, q.q, q.nq);
+  for (int i = 0; i < q.nq; ++i) idx[i] = 1 + i;
   return QS_GEN;
 }
 

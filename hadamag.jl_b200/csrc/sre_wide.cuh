@@ -142,57 +142,6 @@ __device__ __forceinline__ void lane_wht(V (&v)[32], int lane, int m) {
   }
 }
 
-// y^e for integer e >= 1 by repeated squaring, N values side by side
-template <int N>
-__device__ __forceinline__ void powi_many(const double (&y)[N], int e, double (&r)[N]) {
-  double b[N];
-#pragma unroll
-  for (int t = 0; t < N; ++t) b[t] = y[t], r[t] = 1.0;
-  while (e) {
-    if (e & 1) {
-#pragma unroll
-      for (int t = 0; t < N; ++t) r[t] *= b[t];
-    }
-    e >>= 1;
-    if (e) {
-#pragma unroll
-      for (int t = 0; t < N; ++t) b[t] *= b[t];
-    }
-  }
-}
-
-// Generic Renyi indices over the 64 values of a lane, staged in its own 64 slots of shared
-// memory (sm[lane + 32 t]): a rolled loop of four values at a time, so that integer powers
-// and pow() run four independent chains.
-template <typename T>
-__device__ __noinline__ void wide_moments_gen(const T *sm, int lane, double *s, const QParams &qp) {
-  double a2 = 0.0, ag[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 1
-  for (int t0 = 0; t0 < 64; t0 += 4) {
-    double y[4], r[4];
-#pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const double f = (double)sm[lane + 32 * (t0 + t)];
-      y[t] = f * f;
-    }
-    a2 += (y[0] + y[1]) + (y[2] + y[3]);
-#pragma unroll 1
-    for (int k = 0; k < qp.nq; ++k) {
-      const double q = qp.q[k];
-      if (q == floor(q) && q >= 1.0 && q <= 16.0) {
-        powi_many<4>(y, (int)q, r);
-      } else {
-#pragma unroll
-        for (int t = 0; t < 4; ++t) r[t] = pow(y[t], q);
-      }
-      ag[k] += (r[0] + r[1]) + (r[2] + r[3]);
-    }
-  }
-  s[0] = a2;
-#pragma unroll
-  for (int t = 0; t < 4; ++t) s[1 + t] = ag[t];
-}
-
 // Butterflies over the LV low bits of the register index (and, with PAIR, over the bit inside
 // a pair), then the per-lane sums of F^2 and (F^2)^q.
 // q = 2 alone: the last two bits are not transformed (QuadSums).
@@ -231,16 +180,7 @@ __device__ __forceinline__ void wide_moments(V (&v)[32], double *s, const QParam
         v[i].y = a - b;
       }
     }
-    if constexpr (QS == QS_GEN) {
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        sm[lane + 64 * i] = v[i].x;
-        sm[lane + 64 * i + 32] = v[i].y;
-      }
-      wide_moments_gen(sm, lane, s, qp);
-    } else {
-      lane_moments<32, QS>(v, s, qp, (V *)nullptr, lane);  // q = 2 and 3: no staging
-    }
+    lane_moments<32, QS>(v, s, qp, reinterpret_cast<V *>(sm), lane);
   }
 }
 
@@ -316,7 +256,7 @@ __global__ void __launch_bounds__(32 * G, WideOcc<T, G>::value) k_sre_wide(SreAr
     wide_get<T, G>(v, buf, w, lane);
     wide_lane_bits<G>(v, lane);
     double s[NQ + 1];
-    if constexpr (QS == QS_GEN) __syncthreads();  // the moments stage their values in the buffer
+    if (QS == QS_GEN && !a.qp.direct) __syncthreads();  // the moments stage their values in the buffer
     wide_moments<QS, 5, true>(v, s, a.qp, buf + 2048 * w, lane);
     s[0] = x == 0 ? s[0] : 4.0 * s[0];
 #pragma unroll
@@ -451,7 +391,7 @@ __global__ void __launch_bounds__(32 * WideCta<G>::WARPS, (sizeof(T) == 8 ? 8 : 
 #pragma unroll
           for (int m = 1 << CB; m < 32; m <<= 1) lane_wht(v, lane, m);
         }
-        if constexpr (QS == QS_GEN) group_sync<32 * G>(1 + grp);  // the moments stage in the buffer
+        if (QS == QS_GEN && !a.qp.direct) group_sync<32 * G>(1 + grp);  // the moments stage in the buffer
         wide_moments<QS, (HI <= 5 ? HI : 5), (HI > 5)>(v, s, a.qp, buf + 2048 * w, lane);
         s[0] = x == 0 ? s[0] : 4.0 * s[0];
 #pragma unroll
