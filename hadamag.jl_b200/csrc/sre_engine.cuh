@@ -82,6 +82,19 @@ __device__ __forceinline__ void wht_class(V (&v)[32], int c) {
     if (LO <= 4 && HI > 4 && !(i & 16)) bfly<4>(v, i);
 }
 
+// one transform bit held by lane bit `m` (a mask): every value meets its partner's
+template <int R, typename V>
+__device__ __forceinline__ void lane_wht(V (&v)[R], int lane, int m) {
+  const float s = (lane & m) ? -1.0f : 1.0f;
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const auto px = __shfl_xor_sync(0xffffffffu, v[i].x, m);
+    const auto py = __shfl_xor_sync(0xffffffffu, v[i].y, m);
+    v[i].x = fma(v[i].x, (decltype(px))s, px);
+    v[i].y = fma(v[i].y, (decltype(py))s, py);
+  }
+}
+
 // layout A -> layout B through a warp-private buffer of 32R elements
 template <int R, typename V>
 __device__ __forceinline__ void transpose_ab(V (&v)[R], V *sm, int lane) {

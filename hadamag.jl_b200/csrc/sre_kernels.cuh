@@ -78,8 +78,9 @@ __device__ __forceinline__ void fold_last(const SreArgs &a, int nrec) {
 }
 
 // ---------------------------------------------------------------------------------
-// Fused sweep, n - 1 = NB <= PB element bits: one warp holds 2^(PB - NB) X-strings
-// (consecutive Gray indices), builds, transforms and reduces them without leaving the SM.
+// Fused sweep, n - 1 = NB <= PB = 5 + log2 R element bits: one warp holds 2^(PB - NB)
+// X-strings (consecutive Gray indices), builds, transforms and reduces them without leaving
+// the SM.  R < 32: bits log2 R .. 4 run on lane bits after the transpose.
 // The state is always read in FP64 and f = conj(psi(r)) psi(r ^ x) is formed in FP64;
 // the FP32 variant rounds f, not psi, so that its error stays second order.
 template <typename T, int R, int NB, int QS>
@@ -128,7 +129,9 @@ __global__ void __launch_bounds__(FUSED_WARPS * 32) k_sre_fused(SreArgs a) {
     }
     if constexpr (NB > 5) reg_wht<R, 0, NB - 5>(v);
     transpose_ab<R>(v, sm, lane);
-    reg_wht<R, 0, (NB < 5 ? NB : 5)>(v);
+    reg_wht<R, 0, (NB < LOGR ? NB : LOGR)>(v);
+#pragma unroll
+    for (int b = LOGR; b < (NB < 5 ? NB : 5); ++b) lane_wht(v, lane, 1 << (b - LOGR));
     double s[NQ + 1];
     lane_moments<R, QS>(v, s, a.qp, sm, lane);
     if (LANE_UNIFORM) {

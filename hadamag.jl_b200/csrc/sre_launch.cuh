@@ -367,9 +367,18 @@ static int launch_stages3(hm_ctx *c, const SreArgs &a0, int *nwarps_out) {
   return HM_OK;
 }
 
+// Complex registers per lane of k_sre_fused.  Up to n = 10 the 2^n X-strings do not fill the
+// SMs' warps and a warp's serial chain is the kernel's time, so a warp takes as few of them
+// as keeps bits 5 and up in registers (bits 3 and 4 go to lane bits).  At n = 11 a warp per
+// X-string fills them: FP64 takes the single-CTA kernel with one warp, whose exchange is
+// half as wide; FP32 keeps the 32 registers.  SRE call of q = 2, FP64 on B200, 32 registers
+// everywhere -> this: n = 6 41.7 -> 37.8 us, 8 38.9 -> 34.0, 9 39.0 -> 36.7, 10 41.6 -> 40.0,
+// 11 55.7 -> 47.3.
+constexpr int fused_regs(int nb) { return nb <= 8 ? 8 : nb == 9 ? 16 : 32; }
+
 #define HM_FUSED_CASE(NBv)                                         \
   case NBv:                                                        \
-    return launch_fused<T, R, ((NBv) <= PB ? (NBv) : PB), QS>(c, a, nw);
+    return launch_fused<T, fused_regs(NBv), NBv, QS>(c, a, nw);
 template <typename T, int R, int QS>
 static int dispatch_sre(hm_ctx *c, const SreArgs &a, int *nw) {
   constexpr int PB = ilog2c(R) + 5;
@@ -386,8 +395,11 @@ static int dispatch_sre(hm_ctx *c, const SreArgs &a, int *nw) {
       HM_FUSED_CASE(7)
       HM_FUSED_CASE(8)
       HM_FUSED_CASE(9)
-      HM_FUSED_CASE(10)
-      HM_FUSED_CASE(11)
+      case 10:
+        if constexpr (sizeof(T) == 8)
+          return launch_wide<T, 1, QS>(c, a, nw);
+        else
+          return launch_fused<T, 32, 10, QS>(c, a, nw);
       default:
         break;
     }

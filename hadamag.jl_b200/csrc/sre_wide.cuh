@@ -1,6 +1,7 @@
-// sre_wide.cuh -- exact-SRE transforms held by a group of G warps (G = 2, 4, 8, in FP32 also
-// 16): the whole transform of an X-string for n = 12, 13, 14 (FP32 also 15; 2^(n-1) = 1024 G
-// complex values) without leaving the SM, and the two-pass sweep of larger n.
+// sre_wide.cuh -- exact-SRE transforms held by a group of G warps (G = 2, 4, 8; in FP64 also
+// 1, in FP32 also 16): the whole transform of an X-string for n = 12, 13, 14 (FP64 also 11,
+// FP32 15; 2^(n-1) = 1024 G complex values) without leaving the SM, and the two-pass sweep
+// of larger n.
 //
 // The WHT is real-linear, so the real and imaginary parts separate after the products:
 //   phase A  lane l, register i of warp w holds the complex element e = 32 i + l + 1024 w:
@@ -18,7 +19,7 @@
 //   q = 2   FP64  n = 12: 69 -> 31   n = 13: 226 -> 124   n = 14: 1107 -> 530
 //           FP32  n = 12: 60 -> 32   n = 13: 144 -> 81    n = 14: 614 -> 308
 //                 n = 15: 2180 -> 1430 (2030 with the two-pass sweep below)
-//   n = 13, FP64: q = 2 and 3 231 -> 137, q = 4 724 -> 291, q = 2.5 1498 -> 1032
+//   n = 13, FP64: q = 2 and 3 231 -> 137, q = 4 724 -> 155, q = 2.5 1498 -> 155
 // FP64 at n = 13 is 1.04 clocks per complex element and SM, 0.55 of them FP64 issue.
 #pragma once
 #include "sre_kernels.cuh"
@@ -59,13 +60,14 @@ __device__ __forceinline__ void wide_put(V (&v)[32], T *buf, int w, int lane) {
 
 // Element bits of a phase-B lane that are not in its registers: five on the lane number, the
 // rest (with the plane as the top one) on the warp number.
+//   G = 1: lanes 5 6 7 8 9,     the plane in the registers, where larger G have bit 10
 //   G = 2: lanes 5 6 7 8 9,     warp: plane
 //   G = 4: lanes 5 6 7 8 11,    warp: 9, plane
 //   G = 8: lanes 5 6 7 11 12,   warp: 8, 9, plane
 //   G = 16: lanes 5 6 11 12 13, warp: 7, 8, 9, plane
 template <int G>
 __device__ __forceinline__ uint32_t wide_base(int w, int lane) {
-  if constexpr (G == 2) {
+  if constexpr (G <= 2) {
     return (uint32_t)lane << 5;
   } else if constexpr (G == 4) {
     return ((uint32_t)(lane & 15) << 5) | ((uint32_t)(lane >> 4) << 11) | ((uint32_t)(w & 1) << 9);
@@ -80,7 +82,7 @@ __device__ __forceinline__ uint32_t wide_base(int w, int lane) {
 // 0 inside the pair
 template <typename T, int G, typename V>
 __device__ __forceinline__ void wide_get(V (&v)[32], const T *buf, int w, int lane) {
-  const T *plane = buf + (w >= G / 2 ? 1024 * G : 0);
+  const T *plane = buf + (G > 1 && w >= G / 2 ? 1024 * G : 0);
   const uint32_t base = wide_base<G>(w, lane);
 #pragma unroll
   for (int b = 0; b < 2; ++b) {
@@ -127,19 +129,6 @@ __device__ __forceinline__ void wide_unput(V (&v)[32], const T *buf, int w, int 
   }
 #pragma unroll
   for (int c = 0; c < 4; ++c) wht_class<2, 5>(v, c);
-}
-
-// one transform bit held by lane bit `m` (a mask): every value meets its partner's
-template <typename V>
-__device__ __forceinline__ void lane_wht(V (&v)[32], int lane, int m) {
-  const float s = (lane & m) ? -1.0f : 1.0f;
-#pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    const auto px = __shfl_xor_sync(0xffffffffu, v[i].x, m);
-    const auto py = __shfl_xor_sync(0xffffffffu, v[i].y, m);
-    v[i].x = fma(v[i].x, (decltype(px))s, px);
-    v[i].y = fma(v[i].y, (decltype(py))s, py);
-  }
 }
 
 // Butterflies over the LV low bits of the register index (and, with PAIR, over the bit inside
@@ -257,7 +246,7 @@ __global__ void __launch_bounds__(32 * G, WideOcc<T, G>::value) k_sre_wide(SreAr
     wide_lane_bits<G>(v, lane);
     double s[NQ + 1];
     if (QS == QS_GEN && !a.qp.direct) __syncthreads();  // the moments stage their values in the buffer
-    wide_moments<QS, 5, true>(v, s, a.qp, buf + 2048 * w, lane);
+    wide_moments<QS, (G > 1 ? 5 : 4), true>(v, s, a.qp, buf + 2048 * w, lane);
     s[0] = x == 0 ? s[0] : 4.0 * s[0];
 #pragma unroll
     for (int t = 0; t < NQ; ++t) s[1 + t] *= q_scale<QS>(t, x == 0, a.qp);
