@@ -31,6 +31,7 @@ struct AdjArgs {
   double2 *ring;     // chunk x 2^(n-1)   (two-pass intermediate)
   double2 *G;        // chunk x 2^n
   double2 *grad;     // 2^n, accumulated dm/dpsi
+  double2 *gpart;    // n <= 14: the gather's partial gradients, one per split of the X-strings
   double *mpart;     // per warp: sum (F^2)^q (plain), folded at the end
   double q, cq_x, cq_0, q4;
   int n, U, chunk;
@@ -55,14 +56,14 @@ __device__ __forceinline__ double powi7(double y, int e) {
 // Q = 2, 3: compile-time exponent, unrolled over the registers; Q = 0: q at run time
 // (1 <= q <= 8), in a rolled loop over the lane's own slots of the warp's shared buffer
 // (an unrolled sweep of the run-time power spills registers).
-template <int Q>
-__device__ __forceinline__ double adj_pointwise(double2 (&v)[R], int q, double cq, double2 *sm, int lane) {
+template <int Q, int NR>
+__device__ __forceinline__ double adj_pointwise(double2 (&v)[NR], int q, double cq, double2 *sm, int lane) {
   if constexpr (Q == 0) {
 #pragma unroll
-    for (int i = 0; i < R; ++i) sm[lane + 32 * i] = v[i];
+    for (int i = 0; i < NR; ++i) sm[lane + 32 * i] = v[i];
     double m = 0.0;
 #pragma unroll 1
-    for (int i = 0; i < R; ++i) {
+    for (int i = 0; i < NR; ++i) {
       double2 w = sm[lane + 32 * i];
       const double a2 = w.x * w.x, b2 = w.y * w.y;
       const double pa = powi7(a2, q - 1), pb = powi7(b2, q - 1);
@@ -72,13 +73,13 @@ __device__ __forceinline__ double adj_pointwise(double2 (&v)[R], int q, double c
       sm[lane + 32 * i] = w;
     }
 #pragma unroll
-    for (int i = 0; i < R; ++i) v[i] = sm[lane + 32 * i];
+    for (int i = 0; i < NR; ++i) v[i] = sm[lane + 32 * i];
     __syncwarp();  // the buffer is rewritten by the next transpose
     return m;
   } else {
     double m0 = 0.0, m1 = 0.0;
 #pragma unroll
-    for (int i = 0; i < R; ++i) {
+    for (int i = 0; i < NR; ++i) {
       const double a = v[i].x, b = v[i].y;
       const double a2 = a * a, b2 = b * b;
       const double pa = Q == 2 ? a2 : a2 * a2, pb = Q == 2 ? b2 : b2 * b2;  // (W^2)^(q-1)
@@ -92,16 +93,17 @@ __device__ __forceinline__ double adj_pointwise(double2 (&v)[R], int q, double c
 }
 
 // layout B -> layout A (inverse of transpose_ab)
-__device__ __forceinline__ void transpose_ba(double2 (&v)[R], double2 *sm, int lane) {
-  constexpr int LOGR = 5, SW = 7;
+template <int NR>
+__device__ __forceinline__ void transpose_ba(double2 (&v)[NR], double2 *sm, int lane) {
+  constexpr int LOGR = ilog2c(NR), SW = 7;
 #pragma unroll
-  for (int i = 0; i < R; ++i) {
-    const int e = lane * R + i;
+  for (int i = 0; i < NR; ++i) {
+    const int e = lane * NR + i;
     sm[e ^ ((e >> LOGR) & SW)] = v[i];
   }
   __syncwarp();
 #pragma unroll
-  for (int i = 0; i < R; ++i) {
+  for (int i = 0; i < NR; ++i) {
     const int e = i * 32 + lane;
     v[i] = sm[e ^ ((e >> LOGR) & SW)];
   }
@@ -120,54 +122,50 @@ __device__ __forceinline__ void put_G(double2 *Gx, uint64_t u1, uint64_t u2, dou
 }
 
 // ---------------------------------------------------------------------------------
-// n <= 11: one warp per X-string does everything
-template <int NB>
+// n <= 10: one warp per X-string, forward and backward in the 32 NR >= 2^NB slots of its lanes
+// (bits log2 NR .. 4 on lane bits, see k_sre_fused).  Gamma leaves as from
+// k_adj_wide.  Bound by the serial chain of a warp: there are fewer than the SMs hold.
+template <int NB, int QA>
 __global__ void __launch_bounds__(128) k_adj_fused(AdjArgs a) {
-  extern __shared__ __align__(16) unsigned char smraw[];
+  constexpr int NR = NB <= 8 ? 8 : 16, LOGR = ilog2c(NR), LO = NB < LOGR ? NB : LOGR;
+  __shared__ double2 smbuf[4][32 * NR];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double2 *sm = reinterpret_cast<double2 *>(smraw) + warp * 32 * R;
+  double2 *sm = smbuf[warp];
   const int xi = blockIdx.x * 4 + warp;
-  double mloc = 0.0;
-  if (xi < a.nx) {
-    const uint64_t x = a.x0 + xi;
-    const bool xz = (x == 0);
-    const int j = xz ? NB : 63 - __clzll((long long)x);
-    double2 v[R];
+  allow_next_grid();
+  if (xi >= a.nx) return;
+  const uint32_t x = (uint32_t)xi, up = x == 0 ? 0u : ~((1u << (31 - __clz((int)x))) - 1u);
+  double2 v[NR];
 #pragma unroll
-    for (int i = 0; i < R; ++i) {
-      const uint32_t e = (uint32_t)(i * 32 + lane);
-      double2 f = make_double2(0.0, 0.0);
-      if (e < (1u << NB)) {
-        if (xz)
-          f = zero_pair(a.psi[e], a.psi[e + (1u << NB)]);
-        else {
-          const uint64_t r = insert0(e, j);
-          f = conj_mul(a.psi[r], a.psi[r ^ x]);
-        }
-      }
-      v[i] = f;
-    }
-    if constexpr (NB > 5) reg_wht<R, 0, NB - 5>(v);
-    transpose_ab<R>(v, sm, lane);
-    reg_wht<R, 0, (NB < 5 ? NB : 5)>(v);
-    const int qi = (int)a.q;
-    mloc = adj_pointwise<0>(v, qi, xz ? a.cq_0 : a.cq_x, sm, lane) * (xz ? 1.0 : scalbn(1.0, 2 * (int)a.q));
-    reg_wht<R, 0, (NB < 5 ? NB : 5)>(v);
-    transpose_ba(v, sm, lane);
-    if constexpr (NB > 5) reg_wht<R, 0, NB - 5>(v);
-    double2 *Gx = a.G + (size_t)xi * ((size_t)1 << a.n);
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-      const uint32_t e = (uint32_t)(i * 32 + lane);
-      if (e < (1u << NB)) {
-        const uint64_t u1 = xz ? e : insert0(e, j);
-        const uint64_t u2 = xz ? e + (1u << NB) : (u1 ^ x);
-        put_G(Gx, u1, u2, v[i], xz);
-      }
-    }
+  for (int i = 0; i < NR; ++i) {
+    const uint32_t e = (uint32_t)(i * 32 + lane), r = e + (e & up);
+    double2 f = make_double2(0.0, 0.0);
+    if (e < (1u << NB))
+      f = x == 0 ? zero_pair(ld_psi(a.psi + e), ld_psi(a.psi + e + (1u << NB)))
+                 : conj_mul(ld_psi(a.psi + r), ld_psi(a.psi + (r ^ x)));
+    v[i] = f;
   }
-  mloc = warp_sum(mloc);
-  if (lane == 0) a.mpart[blockIdx.x * 4 + warp] += mloc;
+  auto lane_bits = [&] {
+#pragma unroll
+    for (int b = LOGR; b < (NB < 5 ? NB : 5); ++b) lane_wht(v, lane, 1 << (b - LOGR));
+  };
+  if constexpr (NB > 5) reg_wht<NR, 0, NB - 5>(v);
+  transpose_ab<NR>(v, sm, lane);
+  reg_wht<NR, 0, LO>(v);
+  lane_bits();
+  double m = adj_pointwise<QA>(v, (int)a.q, x == 0 ? a.cq_0 : a.cq_x, sm, lane) * (x == 0 ? 1.0 : a.q4);
+  lane_bits();
+  reg_wht<NR, 0, LO>(v);
+  transpose_ba(v, sm, lane);
+  if constexpr (NB > 5) reg_wht<NR, 0, NB - 5>(v);
+  double2 *gam = a.G + ((size_t)xi << NB);
+#pragma unroll
+  for (int i = 0; i < NR; ++i) {
+    const uint32_t e = (uint32_t)(i * 32 + lane);
+    if (e < (1u << NB)) __stcg(gam + e, v[i]);
+  }
+  m = warp_sum(m);
+  if (lane == 0) a.mpart[xi] = m;
 }
 
 // ---------------------------------------------------------------------------------
@@ -361,7 +359,7 @@ __global__ void __launch_bounds__(32 * ACC_SEGS) k_adj_acc(AdjArgs a) {
 }
 
 // ---------------------------------------------------------------------------------
-// n = 12, 13, 14: one CTA of G = 2^(n-11) warps runs an X-string forward and backward
+// n = 11 .. 14: one CTA of G = 2^(n-11) warps runs an X-string forward and backward
 // without leaving the SM: the forward half of k_sre_wide (sre_wide.cuh), the pointwise map on
 // the real values of phase B, the same levels again (the WHT is its own transpose), and
 // the exchange back into phase A's layout.  Only Gamma leaves, 2^(n-1) complex per X-string in
@@ -376,6 +374,7 @@ __global__ void __launch_bounds__(32 * G, 8 / G) k_adj_wide(AdjArgs a) {
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t e0 = 1024u * w + lane;
   double msum = 0.0;
+  allow_next_grid();
   for (int xi = blockIdx.x; xi < a.nx; xi += gridDim.x) {
     const uint32_t x = (uint32_t)a.x0 + xi;
     double2 v[R];
@@ -389,7 +388,7 @@ __global__ void __launch_bounds__(32 * G, 8 / G) k_adj_wide(AdjArgs a) {
 #pragma unroll
       for (int b = 0; b < 8; ++b) wht_block<0, 2>(v, b);
 #pragma unroll
-      for (int c = 0; c < 4; ++c) wht_class<2, 5>(v, c);
+      for (int c = 0; c < 4; ++c) wht_class<2, (G > 1 ? 5 : 4)>(v, c);  // G = 1: the planes apart
 #pragma unroll
       for (int i = 0; i < R; ++i) {
         const double p = v[i].x, q = v[i].y;
@@ -415,6 +414,7 @@ __global__ void __launch_bounds__(32 * G, 8 / G) k_adj_wide(AdjArgs a) {
     wide_unget<double, G>(v, buf, w, lane);  // each lane's own addresses
     __syncthreads();
     wide_unput<double, G>(v, buf, w, lane);
+    wait_prior_grid();  // the gather of the batch before has read its Gamma
     double2 *gam = a.G + (size_t)xi * HALF + e0;
 #pragma unroll
     for (int i = 0; i < R; ++i) __stcg(gam + 32 * i, v[i]);
@@ -425,16 +425,22 @@ __global__ void __launch_bounds__(32 * G, 8 / G) k_adj_wide(AdjArgs a) {
 
 // grad(u) += sum over the batch's X-strings of G_x(u) psi(u ^ x), G_x from Gamma_x in element
 // order: with j the highest set bit of x, u or (u's bit j set) u ^ x is the element whose
-// bit j is 0, and dropping that bit gives its place.  Work split and order as k_adj_acc.
+// bit j is 0, and dropping that bit gives its place.  Work split and order as k_adj_acc, with
+// the X-strings split over blockIdx.y as well, each split into a gradient of its own (the
+// finishing kernel adds them in order): 2^n / 32 blocks alone leave SMs idle below n = 14 and
+// run long chains of dependent loads (n = 11: 64 blocks of 256 X-strings a warp).
 __global__ void __launch_bounds__(32 * ACC_SEGS) k_adj_gather(AdjArgs a) {
   constexpr int U = 8;  // X-strings' loads in flight per lane
   __shared__ double2 part[ACC_SEGS][32];
   const uint32_t len = 1u << a.n, half = len >> 1;
   const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5;
-  const int per = (a.nx + ACC_SEGS - 1) / ACC_SEGS;
-  const int xb = min(a.nx, seg * per), xe = min(a.nx, xb + per);
+  allow_next_grid();  // the next batch's kernel runs up to its first store of Gamma
+  wait_prior_grid();  // this batch's Gamma
+  const int nseg = ACC_SEGS * gridDim.y, per = (a.nx + nseg - 1) / nseg;
+  const int xb = min(a.nx, (int)(blockIdx.y * ACC_SEGS + seg) * per), xe = min(a.nx, xb + per);
+  double2 *out = a.gpart + (size_t)blockIdx.y * len;
   for (uint32_t base = blockIdx.x * 32u; base < len; base += gridDim.x * 32u) {
-    const uint32_t u = base + lane;
+    const uint32_t u = (base + lane) & (len - 1);  // n < 5: lanes past 2^n repeat the first ones
     double gr[4] = {0.0, 0.0, 0.0, 0.0}, gi[4] = {0.0, 0.0, 0.0, 0.0};
     // x != 0: Gamma_x at u's place, conjugated when u is the first of the pair
     auto load = [&](int xi, double2 &g, double2 &p) {
@@ -479,20 +485,22 @@ __global__ void __launch_bounds__(32 * ACC_SEGS) k_adj_gather(AdjArgs a) {
         sum.x += part[k][lane].x;
         sum.y += part[k][lane].y;
       }
-      double2 o = a.grad[u];
-      o.x += sum.x;
-      o.y += sum.y;
-      a.grad[u] = o;
+      if (a.x0 > 0) {
+        const double2 o = out[u];
+        sum.x += o.x;
+        sum.y += o.y;
+      }
+      if (base + lane < len) out[u] = sum;
     }
     __syncthreads();
   }
 }
 
 // Every block adds up the moment partials in the same order (so all hold the same m), then
-// scales its part of the gradient: one block alone took 57 us at n = 14 and four times that
+// scales its part of the gradient (the sum of its nparts > 0 partial ones): one block alone took 57 us at n = 14 and four times that
 // for every two qubits more.
-__global__ void __launch_bounds__(256) k_adj_finish(double2 *grad, uint64_t len, const double *mpart, int nw,
-                                                    double *m_out) {
+__global__ void __launch_bounds__(256) k_adj_finish(double2 *grad, const double2 *gpart, int nparts, uint64_t len,
+                                                    const double *mpart, int nw, double *m_out) {
   __shared__ double sh[256];
   double s = 0.0;
   for (int i = threadIdx.x; i < nw; i += blockDim.x) s += mpart[i];
@@ -505,7 +513,12 @@ __global__ void __launch_bounds__(256) k_adj_finish(double2 *grad, uint64_t len,
   const double m = sh[0];
   const double scale = -1.0 / (m * 0.69314718055994530942);
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < len; i += (uint64_t)gridDim.x * blockDim.x) {
-    double2 g = grad[i];
+    double2 g = nparts > 0 ? gpart[i] : grad[i];
+    for (int k = 1; k < nparts; ++k) {
+      const double2 p = gpart[(size_t)k * len + i];
+      g.x += p.x;
+      g.y += p.y;
+    }
     grad[i] = make_double2(g.x * scale, g.y * scale);
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) *m_out = m;
@@ -918,11 +931,12 @@ int run_adj_stages(hm_ctx *c, const double2 *psi, int n, int q, double2 *grad, d
 }  // namespace
 
 // scale the gradient by -1 / (m ln 2) and read m back
-static int adj_results(hm_ctx *c, double2 *grad_dev, uint64_t len, const double *mpart, int nslots, double *m_out) {
+static int adj_results(hm_ctx *c, double2 *grad_dev, const double2 *gpart, int nparts, uint64_t len,
+                       const double *mpart, int nslots, double *m_out) {
   HM_CUDA(c, cudaEventRecord(c->ev1, c->stream));
   HM_TRY(ensure_dev(c, (void **)&c->d_out, &c->out_cap, sizeof(double) * 16));
   k_adj_finish<<<(unsigned)std::max<uint64_t>(1, std::min<uint64_t>(len / 256, 2 * (uint64_t)c->num_sms)), 256, 0,
-                 c->stream>>>(grad_dev, len, mpart, nslots, c->d_out);
+                 c->stream>>>(grad_dev, gpart, nparts, len, mpart, nslots, c->d_out);
   c->launches += 1;
   HM_TRY(ensure_host(c, (void **)&c->h_out, &c->h_out_cap, sizeof(double) * 24));
   HM_CUDA(c, cudaMemcpyAsync(c->h_out, c->d_out, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -934,11 +948,55 @@ static int adj_results(hm_ctx *c, double2 *grad_dev, uint64_t len, const double 
   return HM_OK;
 }
 
-// n = 12, 13, 14: batches of whole rounds of k_adj_wide's CTAs, each followed by its share of
-// the gradient.  Three rounds make 57 MB of Gamma, which the gather finds in L2: n = 14
-// 2.05 ms of kernels; with two rounds 2.28 (more launches), with four 2.26 (Gamma leaves
-// L2).  The four-kernel stages took 2.68 (n = 12: 0.27 -> 0.22, n = 13: 0.78 -> 0.60).
+// n <= 14: batches of X-strings, Gamma (k_adj_fused, k_adj_wide) and its share of the gradient
+// (k_adj_gather).  n <= 10 is one batch; above, three whole rounds of k_adj_wide's CTAs make
+// 57 MB of Gamma, which the gather finds in L2: n = 14 1.88 ms of kernels; with two rounds 1.96
+// (more launches), with four 2.06 (Gamma leaves L2); unchained launches 2.12.  Against one
+// block per 32 entries for the gather, both partners' Gamma stored and, n <= 11, 32 registers
+// per lane (us of kernels): n = 8 24 -> 15, 9 34 -> 14, 10 57 -> 16, 11 112 -> 33,
+// 12 214 -> 108, 13 599 -> 435.
 static constexpr int wide_rounds = 3;
+
+struct AdjBatches {
+  int nslots, batch, splits;
+};
+
+// buffers of the batches; splits: enough blocks for the SMs (512; n = 13 435 us, with 1024 440,
+// with 2048 461), each warp of the gather keeping at least one round of eight X-strings
+static int adj_prepare(hm_ctx *c, AdjArgs &a, AdjBatches &b) {
+  const uint64_t len = 1ull << a.n;
+  b.splits = 1;
+  while (len / 32 * b.splits < 512 && b.batch / (2 * b.splits * ACC_SEGS) >= 8) b.splits *= 2;
+  HM_TRY(ensure_dev(c, &c->d_inter, &c->inter_cap, ((size_t)b.batch * (len / 2) + b.splits * len) * sizeof(double2)));
+  a.G = (double2 *)c->d_inter;
+  a.gpart = a.G + (size_t)b.batch * (len / 2);
+  HM_TRY(ensure_dev(c, (void **)&c->d_partials, &c->partials_cap, b.nslots * sizeof(double)));
+  a.mpart = c->d_partials;
+  return HM_OK;
+}
+
+// The kernels of the batches are chained by programmatic dependent launch (the first one
+// waits for all before it): each waits for its predecessor before its first access that
+// depends on it, and so for all earlier ones.
+static cudaError_t adj_launch(hm_ctx *c, void (*kern)(AdjArgs), dim3 grid, int threads, size_t smem, bool chained,
+                              const AdjArgs &a) {
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = grid;
+  lc.blockDim = dim3(threads);
+  lc.dynamicSmemBytes = smem;
+  lc.stream = c->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = at;
+  lc.numAttrs = chained ? 1 : 0;
+  c->launches += 1;
+  return cudaLaunchKernelEx(&lc, kern, a);
+}
+
+static cudaError_t adj_gather(hm_ctx *c, const AdjArgs &a, const AdjBatches &b) {
+  return adj_launch(c, k_adj_gather, dim3(std::max(1u, (1u << a.n) / 32), b.splits), 32 * ACC_SEGS, 0, true, a);
+}
 
 template <int G>
 static int launch_adj_wide(hm_ctx *c, AdjArgs &a, double *m_out, double2 *grad_dev) {
@@ -947,29 +1005,46 @@ static int launch_adj_wide(hm_ctx *c, AdjArgs &a, double *m_out, double2 *grad_d
   auto kern = a.q == 2.0 ? k_adj_wide<G, 2> : a.q == 3.0 ? k_adj_wide<G, 3> : k_adj_wide<G, 0>;
   int occ = 0;
   HM_TRY(kernel_occ(c, kern, 32 * G, smem, &occ));
-  const int blocks = (int)std::min<uint64_t>(len, (uint64_t)c->num_sms * occ), nslots = blocks * G;
-  const int batch = (int)std::min<uint64_t>(len, (uint64_t)wide_rounds * blocks);
-  HM_TRY(ensure_dev(c, &c->d_inter, &c->inter_cap, (size_t)batch * (len / 2) * sizeof(double2)));
-  a.G = (double2 *)c->d_inter;
-  a.grad = grad_dev;
-  HM_CUDA(c, cudaMemsetAsync(grad_dev, 0, len * sizeof(double2), c->stream));
-  HM_TRY(ensure_dev(c, (void **)&c->d_partials, &c->partials_cap, nslots * sizeof(double)));
-  HM_CUDA(c, cudaMemsetAsync(c->d_partials, 0, nslots * sizeof(double), c->stream));
-  a.mpart = c->d_partials;
+  const int blocks = (int)std::min<uint64_t>(len, (uint64_t)c->num_sms * occ);
+  AdjBatches b{blocks * G, (int)std::min<uint64_t>(len, (uint64_t)wide_rounds * blocks), 1};
+  HM_TRY(adj_prepare(c, a, b));
+  HM_CUDA(c, cudaMemsetAsync(a.mpart, 0, b.nslots * sizeof(double), c->stream));
   HM_CUDA(c, cudaEventRecord(c->ev0, c->stream));
-  for (uint64_t x0 = 0; x0 < len; x0 += batch) {
+  for (uint64_t x0 = 0; x0 < len; x0 += b.batch) {
     a.x0 = x0;
-    a.nx = (int)std::min<uint64_t>(batch, len - x0);
-    kern<<<std::min(blocks, a.nx), 32 * G, smem, c->stream>>>(a);
-    k_adj_gather<<<(unsigned)(len / 32), 32 * ACC_SEGS, 0, c->stream>>>(a);
-    c->launches += 2;
+    a.nx = (int)std::min<uint64_t>(b.batch, len - x0);
+    HM_CUDA(c, adj_launch(c, kern, dim3(std::min(blocks, a.nx)), 32 * G, smem, x0 > 0, a));
+    HM_CUDA(c, adj_gather(c, a, b));
   }
-  HM_CUDA(c, cudaGetLastError());
-  return adj_results(c, grad_dev, len, a.mpart, nslots, m_out);
+  return adj_results(c, grad_dev, a.gpart, b.splits, len, a.mpart, b.nslots, m_out);
 }
 
-static int run_adj_wide(hm_ctx *c, AdjArgs &a, double *m_out, double2 *grad_dev) {
+template <int NB>
+static int launch_adj_fused(hm_ctx *c, AdjArgs &a, double *m_out, double2 *grad_dev) {
+  constexpr int len = 2 << NB;
+  auto kern = a.q == 2.0 ? k_adj_fused<NB, 2> : a.q == 3.0 ? k_adj_fused<NB, 3> : k_adj_fused<NB, 0>;
+  AdjBatches b{len, len, 1};
+  HM_TRY(adj_prepare(c, a, b));
+  a.nx = len;
+  HM_CUDA(c, cudaEventRecord(c->ev0, c->stream));
+  HM_CUDA(c, adj_launch(c, kern, dim3((len + 3) / 4), 128, 0, false, a));
+  HM_CUDA(c, adj_gather(c, a, b));
+  return adj_results(c, grad_dev, a.gpart, b.splits, len, a.mpart, b.nslots, m_out);
+}
+
+static int run_adj_on_chip(hm_ctx *c, AdjArgs &a, double *m_out, double2 *grad_dev) {
   switch (a.n) {
+    case 1: return launch_adj_fused<0>(c, a, m_out, grad_dev);
+    case 2: return launch_adj_fused<1>(c, a, m_out, grad_dev);
+    case 3: return launch_adj_fused<2>(c, a, m_out, grad_dev);
+    case 4: return launch_adj_fused<3>(c, a, m_out, grad_dev);
+    case 5: return launch_adj_fused<4>(c, a, m_out, grad_dev);
+    case 6: return launch_adj_fused<5>(c, a, m_out, grad_dev);
+    case 7: return launch_adj_fused<6>(c, a, m_out, grad_dev);
+    case 8: return launch_adj_fused<7>(c, a, m_out, grad_dev);
+    case 9: return launch_adj_fused<8>(c, a, m_out, grad_dev);
+    case 10: return launch_adj_fused<9>(c, a, m_out, grad_dev);
+    case 11: return launch_adj_wide<1>(c, a, m_out, grad_dev);
     case 12: return launch_adj_wide<2>(c, a, m_out, grad_dev);
     case 13: return launch_adj_wide<4>(c, a, m_out, grad_dev);
     default: return launch_adj_wide<8>(c, a, m_out, grad_dev);
@@ -986,68 +1061,36 @@ int run_sre_grad(hm_ctx *c, const double2 *psi, int n, int q, double *m_out, dou
   a.cq_0 = 2.0 * q;
   a.q4 = pow(4.0, q);
   const uint64_t len = 1ull << n;
-  if (n >= 12 && n <= 14) return run_adj_wide(c, a, m_out, grad_dev);
-  // chunk: G of at most 1 GiB.  Each chunk costs four launches; with small chunks (16
-  // X-strings at n = 18 for 64 MiB) the launches were under-filled and dominated the time
-  int chunk = (int)std::max<uint64_t>(1, ((uint64_t)1 << 30) / (len * sizeof(double2)));
-  if ((uint64_t)chunk > len) chunk = (int)len;
-  if (n >= 12 && chunk > (1 << PB)) chunk = 1 << PB;  // the chunked kernels only see x < 2^PB
+  if (n <= 14) return run_adj_on_chip(c, a, m_out, grad_dev);
+  // x < 2^PB (relabelled copies, x = 0) in chunks: G of at most 1 GiB.  Each chunk costs four
+  // launches; with small chunks (16 X-strings at n = 18 for 64 MiB) the launches were
+  // under-filled and dominated the time.  The stage kernels run the other X-strings.
+  const int x_chunked = 1 << PB;
+  const int chunk = (int)std::min<uint64_t>(x_chunked, ((uint64_t)1 << 30) / (len * sizeof(double2)));
   a.chunk = chunk;
-  HM_TRY(ensure_dev(c, &c->d_inter, &c->inter_cap, (size_t)chunk * len * sizeof(double2) +
-                                                       (n >= 15 ? (size_t)chunk * (len / 2) * sizeof(double2) : 0)));
+  HM_TRY(ensure_dev(c, &c->d_inter, &c->inter_cap, (size_t)chunk * (len + len / 2) * sizeof(double2)));
   a.G = (double2 *)c->d_inter;
   a.ring = a.G + (size_t)chunk * len;
   a.grad = grad_dev;
   HM_CUDA(c, cudaMemsetAsync(grad_dev, 0, len * sizeof(double2), c->stream));
   const size_t smem = 4 * 32 * R * sizeof(double2);
-  int blocks;
-  if (n <= 11) {
-    blocks = (chunk + 3) / 4;
-  } else {
-    a.U = 1 << (n - 11);
-    blocks = (int)(((long long)chunk * a.U + 3) / 4);
-    HM_TRY(ensure_dev(c, &c->d_aux2, &c->aux2_cap, 10 * len * sizeof(double2)));
-    k_psi_swapped<double2><<<c->num_sms * 8, 256, 0, c->stream>>>(psi, (double2 *)c->d_aux2, n, 10);
-    c->launches += 1;
-    for (int j = 0; j < 10; ++j) a.psi_sw[j] = (const double2 *)c->d_aux2 + (size_t)j * len;
-  }
+  a.U = 1 << (n - 11);
+  const int blocks = (int)(((long long)chunk * a.U + 3) / 4);
+  HM_TRY(ensure_dev(c, &c->d_aux2, &c->aux2_cap, 10 * len * sizeof(double2)));
+  k_psi_swapped<double2><<<c->num_sms * 8, 256, 0, c->stream>>>(psi, (double2 *)c->d_aux2, n, 10);
+  c->launches += 1;
+  for (int j = 0; j < 10; ++j) a.psi_sw[j] = (const double2 *)c->d_aux2 + (size_t)j * len;
   const int nw = blocks * 4;
   // moment partials: the chunked kernels' warps, then one slot per warp of the stage kernels
-  const size_t nslots = (size_t)nw + (n >= 12 ? adj_stage_slots(c) : 0);
+  const size_t nslots = (size_t)nw + adj_stage_slots(c);
   HM_TRY(ensure_dev(c, (void **)&c->d_partials, &c->partials_cap, nslots * sizeof(double) + 64));
   HM_CUDA(c, cudaMemsetAsync(c->d_partials, 0, nslots * sizeof(double), c->stream));
   a.mpart = c->d_partials;
   const unsigned accb = (unsigned)std::min<uint64_t>((len + 31) / 32, (uint64_t)c->num_sms * 8);
   HM_CUDA(c, cudaEventRecord(c->ev0, c->stream));
-  // n >= 12: the chunked kernels cover x < 2^PB (relabelled copies, x = 0); the stage
-  // kernels the rest
-  const uint64_t x_chunked = n >= 12 ? std::min<uint64_t>(len, 1u << PB) : len;
-  for (uint64_t x0 = 0; x0 < x_chunked; x0 += chunk) {
+  for (int x0 = 0; x0 < x_chunked; x0 += chunk) {
     a.x0 = x0;
-    a.nx = (int)std::min<uint64_t>(chunk, x_chunked - x0);
-    if (n <= 11) {
-#define HM_ADJF(NBv)                                                                                  \
-  case NBv:                                                                                           \
-    cudaFuncSetAttribute(k_adj_fused<NBv>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);   \
-    k_adj_fused<NBv><<<blocks, 128, smem, c->stream>>>(a);                                            \
-    break;
-      switch (n - 1) {
-        HM_ADJF(0)
-        HM_ADJF(1)
-        HM_ADJF(2)
-        HM_ADJF(3)
-        HM_ADJF(4)
-        HM_ADJF(5)
-        HM_ADJF(6)
-        HM_ADJF(7)
-        HM_ADJF(8)
-        HM_ADJF(9)
-        HM_ADJF(10)
-        default:
-          break;
-      }
-#undef HM_ADJF
-    } else {
+    a.nx = std::min(chunk, x_chunked - x0);
 #define HM_ADJP(HIv)                                                                              \
   case HIv:                                                                                       \
     cudaFuncSetAttribute(k_adj_p1<HIv>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
@@ -1057,28 +1100,25 @@ int run_sre_grad(hm_ctx *c, const double2 *psi, int n, int q, double *m_out, dou
     k_adj_p2<HIv><<<blocks, 128, smem, c->stream>>>(a);                                           \
     k_adj_p1b<HIv><<<blocks, 128, smem, c->stream>>>(a);                                          \
     break;
-      switch (n - 11) {
-        HM_ADJP(4)
-        HM_ADJP(5)
-        HM_ADJP(6)
-        HM_ADJP(7)
-        HM_ADJP(8)
-        HM_ADJP(9)
-        HM_ADJP(10)
-        default:
-          break;
-      }
-#undef HM_ADJP
+    switch (n - 11) {
+      HM_ADJP(4)
+      HM_ADJP(5)
+      HM_ADJP(6)
+      HM_ADJP(7)
+      HM_ADJP(8)
+      HM_ADJP(9)
+      HM_ADJP(10)
+      default:
+        break;
     }
+#undef HM_ADJP
     k_adj_acc<<<accb, 32 * ACC_SEGS, 0, c->stream>>>(a);
-    c->launches += n <= 11 ? 2 : 4;
+    c->launches += 4;
   }
   HM_CUDA(c, cudaGetLastError());
-  if (n >= 12 && len > x_chunked) {
-    int nw_st = 0;
-    HM_TRY(run_adj_stages(c, psi, n, q, grad_dev, c->d_partials + nw, &nw_st));
-  }
-  return adj_results(c, grad_dev, len, a.mpart, (int)nslots, m_out);
+  int nw_st = 0;
+  HM_TRY(run_adj_stages(c, psi, n, q, grad_dev, c->d_partials + nw, &nw_st));
+  return adj_results(c, grad_dev, nullptr, 0, len, a.mpart, (int)nslots, m_out);
 }
 
 }  // namespace hm

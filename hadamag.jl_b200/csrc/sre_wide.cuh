@@ -107,7 +107,7 @@ __device__ __forceinline__ void wide_get(V (&v)[32], const T *buf, int w, int la
 template <typename T, int G, typename V>
 __device__ __forceinline__ void wide_unget(const V (&v)[32], T *buf, int w, int lane) {
   static_assert(sizeof(T) == 8, "FP64 only");
-  T *plane = buf + (w >= G / 2 ? 1024 * G : 0);
+  T *plane = buf + (G > 1 && w >= G / 2 ? 1024 * G : 0);
   const uint32_t base = wide_base<G>(w, lane);
 #pragma unroll
   for (int b = 0; b < 2; ++b)
