@@ -420,7 +420,10 @@ __global__ void __launch_bounds__(32 * G, 8 / G) k_adj_wide(AdjArgs a) {
     for (int i = 0; i < R; ++i) __stcg(gam + 32 * i, v[i]);
   }
   msum = warp_sum(msum);
-  if (lane == 0) a.mpart[blockIdx.x * G + w] += msum;
+  if (lane == 0) {
+    double *slot = a.mpart + blockIdx.x * G + w;
+    *slot = a.x0 == 0 ? msum : *slot + msum;
+  }
 }
 
 // grad(u) += sum over the batch's X-strings of G_x(u) psi(u ^ x), G_x from Gamma_x in element
@@ -930,21 +933,27 @@ int run_adj_stages(hm_ctx *c, const double2 *psi, int n, int q, double2 *grad, d
 
 }  // namespace
 
-// scale the gradient by -1 / (m ln 2) and read m back
-static int adj_results(hm_ctx *c, double2 *grad_dev, const double2 *gpart, int nparts, uint64_t len,
-                       const double *mpart, int nslots, double *m_out) {
+struct AdjResult {
+  double *m;      // host: sum of (F^2)^q
+  double2 *grad;  // device
+  double *host;   // the caller's gradient
+};
+
+// scale the gradient by -1 / (m ln 2) and read both back (m straight into page-locked memory)
+static int adj_results(hm_ctx *c, const AdjResult &o, const double2 *gpart, int nparts, uint64_t len,
+                       const double *mpart, int nslots) {
   HM_CUDA(c, cudaEventRecord(c->ev1, c->stream));
-  HM_TRY(ensure_dev(c, (void **)&c->d_out, &c->out_cap, sizeof(double) * 16));
-  k_adj_finish<<<(unsigned)std::max<uint64_t>(1, std::min<uint64_t>(len / 256, 2 * (uint64_t)c->num_sms)), 256, 0,
-                 c->stream>>>(grad_dev, gpart, nparts, len, mpart, nslots, c->d_out);
-  c->launches += 1;
   HM_TRY(ensure_host(c, (void **)&c->h_out, &c->h_out_cap, sizeof(double) * 24));
-  HM_CUDA(c, cudaMemcpyAsync(c->h_out, c->d_out, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  k_adj_finish<<<(unsigned)std::max<uint64_t>(1, std::min<uint64_t>(len / 256, 2 * (uint64_t)c->num_sms)), 256, 0,
+                 c->stream>>>(o.grad, gpart, nparts, len, mpart, nslots, c->h_out);
+  c->launches += 1;
+  HM_CUDA(c, cudaGetLastError());
+  HM_CUDA(c, cudaMemcpyAsync(o.host, o.grad, len * sizeof(double2), cudaMemcpyDeviceToHost, c->stream));
   HM_CUDA(c, cudaStreamSynchronize(c->stream));
   float ms = 0.f;
   HM_CUDA(c, cudaEventElapsedTime(&ms, c->ev0, c->ev1));
   c->last_ms = ms;
-  *m_out = c->h_out[0];
+  *o.m = c->h_out[0];
   return HM_OK;
 }
 
@@ -999,7 +1008,7 @@ static cudaError_t adj_gather(hm_ctx *c, const AdjArgs &a, const AdjBatches &b) 
 }
 
 template <int G>
-static int launch_adj_wide(hm_ctx *c, AdjArgs &a, double *m_out, double2 *grad_dev) {
+static int launch_adj_wide(hm_ctx *c, AdjArgs &a, const AdjResult &o) {
   const uint64_t len = 2048ull * G;
   const size_t smem = 2048 * G * sizeof(double);
   auto kern = a.q == 2.0 ? k_adj_wide<G, 2> : a.q == 3.0 ? k_adj_wide<G, 3> : k_adj_wide<G, 0>;
@@ -1008,7 +1017,6 @@ static int launch_adj_wide(hm_ctx *c, AdjArgs &a, double *m_out, double2 *grad_d
   const int blocks = (int)std::min<uint64_t>(len, (uint64_t)c->num_sms * occ);
   AdjBatches b{blocks * G, (int)std::min<uint64_t>(len, (uint64_t)wide_rounds * blocks), 1};
   HM_TRY(adj_prepare(c, a, b));
-  HM_CUDA(c, cudaMemsetAsync(a.mpart, 0, b.nslots * sizeof(double), c->stream));
   HM_CUDA(c, cudaEventRecord(c->ev0, c->stream));
   for (uint64_t x0 = 0; x0 < len; x0 += b.batch) {
     a.x0 = x0;
@@ -1016,11 +1024,11 @@ static int launch_adj_wide(hm_ctx *c, AdjArgs &a, double *m_out, double2 *grad_d
     HM_CUDA(c, adj_launch(c, kern, dim3(std::min(blocks, a.nx)), 32 * G, smem, x0 > 0, a));
     HM_CUDA(c, adj_gather(c, a, b));
   }
-  return adj_results(c, grad_dev, a.gpart, b.splits, len, a.mpart, b.nslots, m_out);
+  return adj_results(c, o, a.gpart, b.splits, len, a.mpart, b.nslots);
 }
 
 template <int NB>
-static int launch_adj_fused(hm_ctx *c, AdjArgs &a, double *m_out, double2 *grad_dev) {
+static int launch_adj_fused(hm_ctx *c, AdjArgs &a, const AdjResult &o) {
   constexpr int len = 2 << NB;
   auto kern = a.q == 2.0 ? k_adj_fused<NB, 2> : a.q == 3.0 ? k_adj_fused<NB, 3> : k_adj_fused<NB, 0>;
   AdjBatches b{len, len, 1};
@@ -1029,29 +1037,29 @@ static int launch_adj_fused(hm_ctx *c, AdjArgs &a, double *m_out, double2 *grad_
   HM_CUDA(c, cudaEventRecord(c->ev0, c->stream));
   HM_CUDA(c, adj_launch(c, kern, dim3((len + 3) / 4), 128, 0, false, a));
   HM_CUDA(c, adj_gather(c, a, b));
-  return adj_results(c, grad_dev, a.gpart, b.splits, len, a.mpart, b.nslots, m_out);
+  return adj_results(c, o, a.gpart, b.splits, len, a.mpart, b.nslots);
 }
 
-static int run_adj_on_chip(hm_ctx *c, AdjArgs &a, double *m_out, double2 *grad_dev) {
+static int run_adj_on_chip(hm_ctx *c, AdjArgs &a, const AdjResult &o) {
   switch (a.n) {
-    case 1: return launch_adj_fused<0>(c, a, m_out, grad_dev);
-    case 2: return launch_adj_fused<1>(c, a, m_out, grad_dev);
-    case 3: return launch_adj_fused<2>(c, a, m_out, grad_dev);
-    case 4: return launch_adj_fused<3>(c, a, m_out, grad_dev);
-    case 5: return launch_adj_fused<4>(c, a, m_out, grad_dev);
-    case 6: return launch_adj_fused<5>(c, a, m_out, grad_dev);
-    case 7: return launch_adj_fused<6>(c, a, m_out, grad_dev);
-    case 8: return launch_adj_fused<7>(c, a, m_out, grad_dev);
-    case 9: return launch_adj_fused<8>(c, a, m_out, grad_dev);
-    case 10: return launch_adj_fused<9>(c, a, m_out, grad_dev);
-    case 11: return launch_adj_wide<1>(c, a, m_out, grad_dev);
-    case 12: return launch_adj_wide<2>(c, a, m_out, grad_dev);
-    case 13: return launch_adj_wide<4>(c, a, m_out, grad_dev);
-    default: return launch_adj_wide<8>(c, a, m_out, grad_dev);
+    case 1: return launch_adj_fused<0>(c, a, o);
+    case 2: return launch_adj_fused<1>(c, a, o);
+    case 3: return launch_adj_fused<2>(c, a, o);
+    case 4: return launch_adj_fused<3>(c, a, o);
+    case 5: return launch_adj_fused<4>(c, a, o);
+    case 6: return launch_adj_fused<5>(c, a, o);
+    case 7: return launch_adj_fused<6>(c, a, o);
+    case 8: return launch_adj_fused<7>(c, a, o);
+    case 9: return launch_adj_fused<8>(c, a, o);
+    case 10: return launch_adj_fused<9>(c, a, o);
+    case 11: return launch_adj_wide<1>(c, a, o);
+    case 12: return launch_adj_wide<2>(c, a, o);
+    case 13: return launch_adj_wide<4>(c, a, o);
+    default: return launch_adj_wide<8>(c, a, o);
   }
 }
 
-int run_sre_grad(hm_ctx *c, const double2 *psi, int n, int q, double *m_out, double2 *grad_dev) {
+static int run_sre_grad(hm_ctx *c, const double2 *psi, int n, int q, const AdjResult &o) {
   AdjArgs a;
   memset(&a, 0, sizeof a);
   a.psi = psi;
@@ -1061,7 +1069,7 @@ int run_sre_grad(hm_ctx *c, const double2 *psi, int n, int q, double *m_out, dou
   a.cq_0 = 2.0 * q;
   a.q4 = pow(4.0, q);
   const uint64_t len = 1ull << n;
-  if (n <= 14) return run_adj_on_chip(c, a, m_out, grad_dev);
+  if (n <= 14) return run_adj_on_chip(c, a, o);
   // x < 2^PB (relabelled copies, x = 0) in chunks: G of at most 1 GiB.  Each chunk costs four
   // launches; with small chunks (16 X-strings at n = 18 for 64 MiB) the launches were
   // under-filled and dominated the time.  The stage kernels run the other X-strings.
@@ -1071,8 +1079,8 @@ int run_sre_grad(hm_ctx *c, const double2 *psi, int n, int q, double *m_out, dou
   HM_TRY(ensure_dev(c, &c->d_inter, &c->inter_cap, (size_t)chunk * (len + len / 2) * sizeof(double2)));
   a.G = (double2 *)c->d_inter;
   a.ring = a.G + (size_t)chunk * len;
-  a.grad = grad_dev;
-  HM_CUDA(c, cudaMemsetAsync(grad_dev, 0, len * sizeof(double2), c->stream));
+  a.grad = o.grad;
+  HM_CUDA(c, cudaMemsetAsync(o.grad, 0, len * sizeof(double2), c->stream));
   const size_t smem = 4 * 32 * R * sizeof(double2);
   a.U = 1 << (n - 11);
   const int blocks = (int)(((long long)chunk * a.U + 3) / 4);
@@ -1117,8 +1125,8 @@ int run_sre_grad(hm_ctx *c, const double2 *psi, int n, int q, double *m_out, dou
   }
   HM_CUDA(c, cudaGetLastError());
   int nw_st = 0;
-  HM_TRY(run_adj_stages(c, psi, n, q, grad_dev, c->d_partials + nw, &nw_st));
-  return adj_results(c, grad_dev, nullptr, 0, len, a.mpart, (int)nslots, m_out);
+  HM_TRY(run_adj_stages(c, psi, n, q, o.grad, c->d_partials + nw, &nw_st));
+  return adj_results(c, o, nullptr, 0, len, a.mpart, (int)nslots);
 }
 
 }  // namespace hm
@@ -1137,9 +1145,7 @@ extern "C" int hm_sre_grad(hm_ctx *c, const double *psi, int n, double q, double
   double2 *dpsi = (double2 *)c->d_psi, *dgrad = dpsi + len;
   HM_CUDA(c, cudaMemcpyAsync(dpsi, psi, len * sizeof(double2), cudaMemcpyHostToDevice, c->stream));
   double m = 0.0;
-  HM_TRY(hm::run_sre_grad(c, dpsi, n, (int)q, &m, dgrad));
-  HM_CUDA(c, cudaMemcpyAsync(grad, dgrad, len * sizeof(double2), cudaMemcpyDeviceToHost, c->stream));
-  HM_CUDA(c, cudaStreamSynchronize(c->stream));
+  HM_TRY(hm::run_sre_grad(c, dpsi, n, (int)q, hm::AdjResult{&m, dgrad, grad}));
   *out_sre = -log2(m / (double)len);
   return HM_OK;
 }
