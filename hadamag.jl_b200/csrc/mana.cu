@@ -339,57 +339,91 @@ struct M9 {
   double2 m[81];
 };
 
-// vec9 (src/Mana.jl:190-228): v[p] = rho[r0 + dim * c0], the base-9 digit of p for site k
-// (site 1 most significant) being 3 i_k + j_k with i_k / j_k the k-th most significant
-// ternary digits of r0 / c0
-__global__ void k_vec_rho(const double2 *__restrict__ rho, double2 *__restrict__ v, int N, int dim, int op) {
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < op; p += gridDim.x * blockDim.x) {
-    int t = p, r0 = 0, c0 = 0, w = 1;
-    for (int k = 0; k < N; ++k) {  // least significant base-9 digit first = site N
-      const int d9 = t % 9;
-      t /= 9;
-      r0 += (d9 / 3) * w;
-      c0 += (d9 % 3) * w;
-      w *= 3;
-    }
-    v[p] = rho[(size_t)r0 + (size_t)dim * c0];
-  }
-}
-
-// one leg of M^{(x)N} (src/Mana.jl:236-281): y = M x on every fiber of stride 9^(N-leg)
-__global__ void k_mana_leg(double2 *v, int op, int stride, M9 M) {
-  const int nfib = op / 9;
-  for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < nfib; f += gridDim.x * blockDim.x) {
-    const int blk = f / stride, ofs = f % stride;
-    const size_t base = (size_t)blk * stride * 9 + ofs;
-    double2 x[9];
-#pragma unroll
-    for (int a = 0; a < 9; ++a) x[a] = v[base + (size_t)a * stride];
-#pragma unroll
-    for (int r = 0; r < 9; ++r) {
-      double sr = 0.0, si = 0.0;
-#pragma unroll
-      for (int c = 0; c < 9; ++c) {
-        const double2 m = M.m[9 * r + c];
-        sr += m.x * x[c].x - m.y * x[c].y;
-        si += m.x * x[c].y + m.y * x[c].x;
+// K of the N legs (9 x 9 phase-point matrices on base-9 digits lg .. lg + K - 1 of the index,
+// least significant first) on tiles of 9^K elements in shared memory, up to 2187 elements a
+// block (`tiles` tiles, fewer where the blocks would not fill the SMs).
+// The first pass reads rho through vec9 (src/Mana.jl:190-228): element p is
+// rho[r0 + dim * c0], the base-9 digit of p for site k (site 1 most significant) being
+// 3 i_k + j_k with i_k / j_k the k-th most significant ternary digits of r0 / c0.  The last
+// pass adds up |w| instead of storing it.  Bound by launches and their drains: one kernel for
+// vec9, each leg and the sum read and wrote 9^N elements N + 2 times.
+// Kernels on B200, that -> this: N = 3 24 -> 14 us, 4 28 -> 16, 5 35 -> 25, 6 55 -> 41.
+constexpr int LEG_BLOCK = 256, LEG_TILE = 2187;
+template <int K>
+__global__ void __launch_bounds__(LEG_BLOCK) k_mana_legs(const double2 *__restrict__ rho, double2 *v, double *slots,
+                                                         int N, int lg, int tiles, M9 M) {
+  constexpr int E = ipow3c(2 * K), FIBERS = E / 9;
+  __shared__ double2 tile[LEG_TILE];
+  __shared__ double red[LEG_BLOCK];
+  const bool first = lg == 0, last = lg + K == N;
+  int dim = 1, S = 1, ntiles = 1;
+  for (int i = 0; i < N; ++i) dim *= 3;
+  for (int i = 0; i < lg; ++i) S *= 9;
+  for (int i = K; i < N; ++i) ntiles *= 9;
+  const int tid = threadIdx.x;
+  double sum = 0.0;
+  for (int t0 = blockIdx.x * tiles; t0 < ntiles; t0 += gridDim.x * tiles) {
+    const int nt = min(tiles, ntiles - t0);
+    // element i of tile t: digits lg .. lg + K - 1 are i, the others t
+    auto place = [&](int t, int i) { return (t / S) * S * E + i * S + t % S; };
+    for (int j = tid; j < nt * E; j += LEG_BLOCK) {
+      if (first) {
+        int p = t0 * E + j, r0 = 0, c0 = 0;
+        for (int k = 0, w = 1; k < N; ++k, w *= 3) {
+          const int d9 = p % 9;
+          p /= 9;
+          r0 += (d9 / 3) * w;
+          c0 += (d9 % 3) * w;
+        }
+        tile[j] = __ldg(rho + (size_t)r0 + (size_t)dim * c0);
+      } else {
+        const int t = j % nt, i = j / nt;  // neighbouring tiles are neighbours in memory
+        tile[t * E + i] = __ldcg(v + place(t0 + t, i));
       }
-      v[base + (size_t)r * stride] = make_double2(sr, si);
     }
-  }
-}
-
-__global__ void k_abs_sum_slots(const double2 *v, int len, double *slots) {
-  __shared__ double red[256];
-  double s = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < len; i += gridDim.x * blockDim.x) s += hypot(v[i].x, v[i].y);
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int stride = k == 0 ? 1 : k == 1 ? 9 : 81;
+      const int f = tid % FIBERS, base = (tid / FIBERS) * E + f / stride * stride * 9 + f % stride;
+      if (tid < nt * FIBERS) {
+        double2 x[9];
+#pragma unroll
+        for (int i = 0; i < 9; ++i) x[i] = tile[base + i * stride];
+#pragma unroll
+        for (int r = 0; r < 9; ++r) {
+          double sr = 0.0, si = 0.0;
+#pragma unroll
+          for (int i = 0; i < 9; ++i) {
+            const double2 m = M.m[9 * r + i];
+            sr += m.x * x[i].x - m.y * x[i].y;
+            si += m.x * x[i].y + m.y * x[i].x;
+          }
+          tile[base + r * stride] = make_double2(sr, si);
+        }
+      }
+      __syncthreads();
+    }
+    for (int j = tid; j < nt * E; j += LEG_BLOCK) {
+      if (last) {
+        sum += hypot(tile[j].x, tile[j].y);
+      } else if (first) {
+        __stcg(v + (size_t)t0 * E + j, tile[j]);
+      } else {
+        const int t = j % nt, i = j / nt;
+        __stcg(v + place(t0 + t, i), tile[t * E + i]);
+      }
+    }
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
+  if (!last) return;
+  red[tid] = sum;
+  __syncthreads();
+  for (int o = LEG_BLOCK / 2; o > 0; o >>= 1) {
+    if (tid < o) red[tid] += red[tid + o];
+    __syncthreads();
+  }
+  if (tid == 0) {
     slots[2 * blockIdx.x] = red[0];
     slots[2 * blockIdx.x + 1] = 0.0;
   }
@@ -522,11 +556,10 @@ static int run_mana_pure_t(hm_ctx *c, const double2 *psi, int xb, int xe, double
   }
   HM_CUDA(c, cudaGetLastError());
   HM_CUDA(c, cudaEventRecord(c->ev1, c->stream));
-  HM_TRY(ensure_dev(c, (void **)&c->d_out, &c->out_cap, sizeof(double) * 16));
-  k_fold_dd<<<1, 256, 0, c->stream>>>(c->d_partials, (int)nslots, c->d_out);
-  c->launches += 1;
   HM_TRY(ensure_host(c, (void **)&c->h_out, &c->h_out_cap, sizeof(double) * 24));
-  HM_CUDA(c, cudaMemcpyAsync(c->h_out, c->d_out, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  k_fold_dd<<<1, 256, 0, c->stream>>>(c->d_partials, (int)nslots, c->h_out);  // page-locked
+  c->launches += 1;
+  HM_CUDA(c, cudaGetLastError());
   HM_CUDA(c, cudaStreamSynchronize(c->stream));
   float ms = 0.f;
   HM_CUDA(c, cudaEventElapsedTime(&ms, c->ev0, c->ev1));
@@ -557,30 +590,35 @@ int run_mana_pure(hm_ctx *c, const double2 *psi, int L, int xb, int xe, double *
 }
 
 int run_mana_mixed(hm_ctx *c, const double2 *rho, int N, double *sum_dd) {
-  const int dim = ipow3(N);
-  int op = 1;
+  size_t op = 1;
   for (int i = 0; i < N; ++i) op *= 9;
-  HM_TRY(ensure_dev(c, &c->d_inter, &c->inter_cap, (size_t)op * sizeof(double2)));
-  double2 *v = (double2 *)c->d_inter;
+  // the legs in the fewest passes of at most three, as even as they come
+  const int passes = (N + 2) / 3;
+  double2 *v = nullptr;
+  if (passes > 1) {
+    HM_TRY(ensure_dev(c, &c->d_inter, &c->inter_cap, op * sizeof(double2)));
+    v = (double2 *)c->d_inter;
+  }
+  const int maxb = c->num_sms * 8;
+  HM_TRY(ensure_dev(c, (void **)&c->d_partials, &c->partials_cap, (size_t)maxb * 2 * sizeof(double)));
+  HM_TRY(ensure_host(c, (void **)&c->h_out, &c->h_out_cap, sizeof(double) * 24));
   const M9 M = phase_point_matrix();
   HM_CUDA(c, cudaEventRecord(c->ev0, c->stream));
-  const int blocks = std::max(1, std::min((op + 255) / 256, c->num_sms * 8));
-  k_vec_rho<<<blocks, 256, 0, c->stream>>>(rho, v, N, dim, op);
-  for (int leg = 1; leg <= N; ++leg) {
-    int stride = 1;
-    for (int i = 0; i < N - leg; ++i) stride *= 9;
-    k_mana_leg<<<std::max(1, std::min((op / 9 + 127) / 128, c->num_sms * 8)), 128, 0, c->stream>>>(v, op, stride, M);
+  int blocks = 1;
+  for (int p = 0, lg = 0; p < passes; ++p) {
+    const int K = (N - lg + passes - p - 1) / (passes - p);
+    const int E = ipow3(2 * K), ntiles = (int)(op / E);
+    const int tiles = std::max(1, std::min(LEG_TILE / E, ntiles / c->num_sms));
+    blocks = std::min((ntiles + tiles - 1) / tiles, maxb);
+    auto kern = K == 3 ? k_mana_legs<3> : K == 2 ? k_mana_legs<2> : k_mana_legs<1>;
+    kern<<<blocks, LEG_BLOCK, 0, c->stream>>>(rho, v, c->d_partials, N, lg, tiles, M);
+    lg += K;
   }
-  const int nb = std::max(1, std::min((op + 255) / 256, c->num_sms * 2));
-  HM_TRY(ensure_dev(c, (void **)&c->d_partials, &c->partials_cap, (size_t)nb * 2 * sizeof(double)));
-  k_abs_sum_slots<<<nb, 256, 0, c->stream>>>(v, op, c->d_partials);
   HM_CUDA(c, cudaGetLastError());
   HM_CUDA(c, cudaEventRecord(c->ev1, c->stream));
-  HM_TRY(ensure_dev(c, (void **)&c->d_out, &c->out_cap, sizeof(double) * 16));
-  k_fold_dd<<<1, 256, 0, c->stream>>>(c->d_partials, nb, c->d_out);
-  c->launches += 3 + N;  // vec9(rho), one per leg, the |w| sums, the fold
-  HM_TRY(ensure_host(c, (void **)&c->h_out, &c->h_out_cap, sizeof(double) * 24));
-  HM_CUDA(c, cudaMemcpyAsync(c->h_out, c->d_out, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  k_fold_dd<<<1, 256, 0, c->stream>>>(c->d_partials, blocks, c->h_out);  // page-locked
+  c->launches += passes + 1;
+  HM_CUDA(c, cudaGetLastError());
   HM_CUDA(c, cudaStreamSynchronize(c->stream));
   float ms = 0.f;
   HM_CUDA(c, cudaEventElapsedTime(&ms, c->ev0, c->ev1));
