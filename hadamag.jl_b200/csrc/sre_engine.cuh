@@ -418,11 +418,37 @@ struct QuadSums {
   }
 };
 
-// q = 2 sums of 32 complex registers whose register bits LO .. 4 are still to transform (bits
-// below 2 done): bit 2 if it is one of them, then quads over bits 3 and 4
-template <int LO, typename V>
+// The same with sum F^6: sum_k (sum_d (-1)^(k.d) c_d)^3 keeps the triples with d1 ^ d2 ^ d3 = 0,
+// 4 (c_0^3 + 3 c_0 (c_1^2 + c_2^2 + c_3^2) + 6 c_1 c_2 c_3).  Here c1 .. c3 are halves of c_1 ..
+// c_3.  21 operations for the four values instead of 8 for the two levels and 20 for the powers.
+// FP64 on B200, q = 2 and 3: n = 13 143 -> 136 us, n = 14 594 -> 547, n = 20 4.00 -> 3.85 each.
+// Error of the q = 3 sum against extended precision, n = 11, 12: 6e-16 (powers: 9e-16).
+struct CubeSums {
+  double a2[2] = {0.0, 0.0}, m4[2] = {0.0, 0.0}, m6[2] = {0.0, 0.0}, m111[2] = {0.0, 0.0};
+  __device__ __forceinline__ void add(int t, double u0, double u1, double u2, double u3) {
+    const double c0 = fma(u0, u0, fma(u1, u1, fma(u2, u2, u3 * u3)));
+    const double c1 = fma(u0, u1, u2 * u3), c2 = fma(u0, u2, u1 * u3), c3 = fma(u0, u3, u1 * u2);
+    const double h = fma(c1, c1, fma(c2, c2, c3 * c3)), w = c0 * c0;
+    a2[t] += c0;
+    m4[t] += fma(4.0, h, w);
+    m6[t] = fma(c0, fma(12.0, h, w), m6[t]);
+    m111[t] = fma(c1 * c2, c3, m111[t]);
+  }
+  __device__ __forceinline__ void get(double *s) const {
+    s[0] = 4.0 * (a2[0] + a2[1]);
+    s[1] = 4.0 * (m4[0] + m4[1]);
+    s[2] = 4.0 * ((m6[0] + m6[1]) + 48.0 * (m111[0] + m111[1]));
+  }
+};
+template <int QS> struct LevelSums;
+template <> struct LevelSums<QS_Q2> : QuadSums {};
+template <> struct LevelSums<QS_Q23> : CubeSums {};
+
+// sums of 32 complex registers whose register bits LO .. 4 are still to transform (bits below
+// 2 done): bit 2 if it is one of them, then quads over bits 3 and 4
+template <int QS, int LO, typename V>
 __device__ __forceinline__ void quad_moments(V (&v)[32], double *s) {
-  QuadSums q;
+  LevelSums<QS> q;
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     if constexpr (LO <= 2) wht_class<2, 3>(v, c);
@@ -673,8 +699,8 @@ __device__ __forceinline__ void p2_unit(const V *__restrict__ tile_ptr, V *sm, i
     for (int b = 0; b < 8; ++b) wht_block<0, 2>(v, b);
     ready();
     wht_exchange<(LOGC < 2 ? LOGC : 2)>(v, sm, lane);
-    if constexpr (QS == QS_Q2 && LOGC <= 3) {
-      quad_moments<LOGC>(v, s);
+    if constexpr ((QS == QS_Q2 || (QS == QS_Q23 && sizeof(V) == 16)) && LOGC <= 3) {
+      quad_moments<QS, LOGC>(v, s);
       return;
     }
 #pragma unroll

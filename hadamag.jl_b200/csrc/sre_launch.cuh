@@ -28,7 +28,7 @@ namespace hm {
 // 2.70, 10.02.  FP64 at n = 20 stays with k_sre_stage (X = 10: 3.74, 3.83 before its q = 2
 // moments by quads; 3.87 here at X = 7): both are bound by the ring's traffic there, and its
 // tensor stores need no group of four.  So does FP64 at n = 19 for q = 2 and 3 together
-// (X = 16: 1.89; 1.91 here).
+// (X = 16: 1.84; 1.89 here at X = 9).
 // hm_autotune measures and records a batch for the machine at hand; setting
 // HM_PARAM_BATCH, _UNITS or _RING switches to the generic rule.
 inline int measured_x(bool fp64, int n) {

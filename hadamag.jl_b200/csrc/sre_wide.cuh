@@ -19,7 +19,7 @@
 //   q = 2   FP64  n = 12: 69 -> 31   n = 13: 226 -> 124   n = 14: 1107 -> 530
 //           FP32  n = 12: 60 -> 32   n = 13: 144 -> 81    n = 14: 614 -> 308
 //                 n = 15: 2180 -> 1430 (2030 with the two-pass sweep below)
-//   n = 13, FP64: q = 2 and 3 231 -> 137, q = 4 724 -> 155, q = 2.5 1498 -> 155
+//   n = 13, FP64: q = 2 and 3 231 -> 136, q = 4 724 -> 155, q = 2.5 1498 -> 155
 // FP64 at n = 13 is 1.04 clocks per complex element and SM, 0.55 of them FP64 issue.
 #pragma once
 #include "sre_kernels.cuh"
@@ -133,14 +133,16 @@ __device__ __forceinline__ void wide_unput(V (&v)[32], const T *buf, int w, int 
 
 // Butterflies over the LV low bits of the register index (and, with PAIR, over the bit inside
 // a pair), then the per-lane sums of F^2 and (F^2)^q.
-// q = 2 alone: the last two bits are not transformed (QuadSums).
+// q = 2 and, in FP64, q = 2 and 3: the last two bits are not transformed (QuadSums, CubeSums;
+// in FP32 the two levels are cheap and the cubes would cost as many FP64 operations as the
+// powers).
 template <int QS, int LV, bool PAIR, typename T, typename V>
 __device__ __forceinline__ void wide_moments(V (&v)[32], double *s, const QParams &qp, T *sm, int lane) {
-  if constexpr (QS == QS_Q2) {
+  if constexpr (QS == QS_Q2 || (QS == QS_Q23 && sizeof(T) == 8)) {
     constexpr int TOP = PAIR ? LV - 1 : LV - 2;  // transformed explicitly: index bits 0 .. TOP-1
 #pragma unroll
     for (int b = 0; b < 8; ++b) wht_block<0, TOP>(v, b);
-    QuadSums quad;
+    LevelSums<QS> quad;
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       wht_class<0, TOP>(v, c);
