@@ -606,11 +606,11 @@ int run_mc(hm_ctx *c, const double2 *psi, int n, double q, int nbeta_grid, int c
   // against 12.1 / 15.1, n = 14 5.3 / 6.2 against 12.1 / 17.2, n = 15 5.7 / 15.5 against
   // 12.6 / 20.7 (601 chains: 71 against 90).  At n = 16 and 17 a chain's cluster takes eight
   // SMs and its exchange crosses them (17 bytes per clock and SM), so that with many chains
-  // the passes through L2 catch up: n = 16 6.9 against 12.5 at 13 chains, 17.4 against 19.5
-  // at 41, 26.7 each at 81; n = 17 10.0 against 16.2 at 13, 20.1 against 21.7 at 21, 30.4
-  // against 29.4 at 41.
+  // the passes through L2 catch up: n = 16 6.9 against 13.0 at 13 chains, 17.0 against 18.5
+  // at 41, 18.6 against 21.4 at 61, 26.7 each at 81.  At n = 17 sixteen clusters are resident
+  // at a time: 10.2 against 17.2 at 15 chains, 19.4 against 17.0 at 17, 20.0 against 19.3 at 21.
   // The rule looks at the whole grid, so that a range of its chains takes the same route.
-  const bool one_launch = n <= 15 || (n == 16 && nbeta_grid <= 64) || (n == 17 && nbeta_grid <= 24);
+  const bool one_launch = n <= 15 || (n == 16 && nbeta_grid <= 64) || (n == 17 && nbeta_grid <= 16);
   if (!one_launch) {
     a.U = 1 << (n - 11);
     HM_TRY(ensure_dev(c, &c->d_inter, &c->inter_cap, (size_t)nbeta * (len / 2) * sizeof(double2)));
