@@ -172,6 +172,8 @@ int sweep_engine(int n, int precision);
 // Exact-SRE raw sums of several states in one persistent launch (12 <= n <= 21 two-pass
 // states and n <= 11 one-warp states); out_dd per item: [p2_hi, p2_lo, m0_hi, m0_lo, ...].
 int run_queue(hm_ctx *c, const QueueItem *items, int nitems, const QReq &q, int precision, double *out_dd);
+// (hi, lo) += (b_hi, b_lo)
+void dd_add_host(double *a, double bh, double bl);
 // as run_queue, with FP32's x = 0 transforms split off into an FP64 launch
 int run_queue_sre(hm_ctx *c, const QueueItem *items, int nitems, const QReq &q, int precision, double *out_dd);
 

@@ -100,7 +100,7 @@ __global__ void k_psi_to_f32(const double2 *__restrict__ in, float2 *__restrict_
 }
 
 // (hi, lo) += (b_hi, b_lo), Knuth TwoSum on the high parts
-static void dd_add_host(double *a, double bh, double bl) {
+void dd_add_host(double *a, double bh, double bl) {
   const double s = a[0] + bh;
   const double bb = s - a[0];
   const double err = (a[0] - (s - bb)) + (bh - bb);
