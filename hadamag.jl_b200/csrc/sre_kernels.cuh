@@ -200,7 +200,12 @@ __global__ void __launch_bounds__(SRE_WARPS * 32, StageOcc<T>::value)
   allow_next_grid();
   // the base only changes between replays, after every node of the replay has finished
   const long long t = (long long)*(volatile unsigned *)a.stage + a.node;
-  if (t > a.nbatch) return;  // padding stages of the last graph replay
+  // padding stages of the last graph replay: they end after the stage that they follow, so that
+  // what comes after the chain (the advance of the base, the fold) finds every stage complete
+  if (t > a.nbatch) {
+    wait_prior_grid();
+    return;
+  }
 #ifdef HM_TMEM_EXCHANGE
   // TMEM for the lane <-> register exchanges (the whole CTA takes part; no return below)
   __shared__ uint32_t tmem_slot;

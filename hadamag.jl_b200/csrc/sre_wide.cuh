@@ -307,7 +307,11 @@ __global__ void __launch_bounds__(32 * WideCta<G>::WARPS, (sizeof(T) == 8 ? 8 : 
   allow_next_grid();
   // the base only changes between replays, after every node of the replay has finished
   const long long t = (long long)*(volatile unsigned *)a.stage + a.node;
-  if (t > a.nbatch) return;  // padding stages of the last graph replay
+  // padding stages of the last graph replay end after the stage that they follow (see k_sre_stage)
+  if (t > a.nbatch) {
+    wait_prior_grid();
+    return;
+  }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int grp = warp / G, w = warp % G;
   T *buf = reinterpret_cast<T *>(smem_wide) + (size_t)grp * ROW;

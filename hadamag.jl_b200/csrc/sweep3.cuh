@@ -137,7 +137,11 @@ __global__ void __launch_bounds__(SRE_WARPS * 32, StageOcc<T>::value)
   V *sm = reinterpret_cast<V *>(smem_stage3) + warp * (32 * R);
   allow_next_grid();
   const long long t = (long long)*(volatile unsigned *)a.stage + a.node;
-  if (t > a.nbatch + 1) return;  // padding stages of the last graph replay
+  // padding stages of the last graph replay end after the stage that they follow (see k_sre_stage)
+  if (t > a.nbatch + 1) {
+    wait_prior_grid();
+    return;
+  }
   const int gwarp = blockIdx.x * SRE_WARPS + warp;
   const int nwarps = gridDim.x * SRE_WARPS;
   const V *psi = reinterpret_cast<const V *>(a.psi);
