@@ -201,22 +201,10 @@ static int enqueue_sweep(hm_ctx *c, const double2 *psi_dev, int n, uint64_t kb, 
   return HM_OK;
 }
 
-// Sweeps of several states one after the other, read back together: every sweep writes its
-// sums to its own page-locked slot, and the host waits once.  FP32: x = 0 (F = WHT of
-// |psi|^2, whose F(0)^4 = 1 can dominate m) is an FP64 sweep of its own, since the FP32
-// kernels would round it; the FP64 kernels build it themselves.
-static int run_sweeps(hm_ctx *c, const QueueItem *items, int nitems, const QReq &q, int precision, double *out_dd) {
-  constexpr int SLOT = 16;
-  QParams qp;
-  int idx[4];
-  const int kind = choose_qs(q, qp, idx);
-  const int nsum = 1 + (kind == QS_Q2 ? 1 : (kind == QS_Q23 ? 2 : 4)), w = 2 * (1 + q.nq);
-  HM_TRY(ensure_host(c, (void **)&c->h_out, &c->h_out_cap, sizeof(double) * 2 * SLOT * (size_t)nitems + 64));
-  if (!c->d_ticket) {
-    HM_CUDA(c, cudaMalloc((void **)&c->d_ticket, 256));
-    HM_CUDA(c, cudaMemsetAsync(c->d_ticket, 0, 256, c->stream));
-  }
-  HM_CUDA(c, cudaEventRecord(c->ev0, c->stream));
+// Queues the sweeps of all items; item i's sums go to the 2 SLOT doubles at i of c->h_out.
+constexpr int SLOT = 16;
+static int enqueue_sweeps(hm_ctx *c, const QueueItem *items, int nitems, int kind, const QParams &qp, int nsum,
+                          int precision) {
   for (int i = 0; i < nitems; ++i) {
     const QueueItem &it = items[i];
     double *slot = c->h_out + (size_t)2 * SLOT * i;
@@ -227,6 +215,31 @@ static int run_sweeps(hm_ctx *c, const QueueItem *items, int nitems, const QReq 
     if (zero) HM_TRY(enqueue_sweep(c, it.psi, it.n, 0, 1, kind, qp, nsum, HM_FP64, slot + SLOT));
   }
   HM_CUDA(c, cudaEventRecord(c->ev1, c->stream));
+  return HM_OK;
+}
+
+// Sweeps of several states one after the other, read back together: every sweep writes its
+// sums to its own page-locked slot, and the host waits once.  FP32: x = 0 (F = WHT of
+// |psi|^2, whose F(0)^4 = 1 can dominate m) is an FP64 sweep of its own, since the FP32
+// kernels would round it; the FP64 kernels build it themselves.
+static int run_sweeps(hm_ctx *c, const QueueItem *items, int nitems, const QReq &q, int precision, double *out_dd) {
+  QParams qp;
+  int idx[4];
+  const int kind = choose_qs(q, qp, idx);
+  const int nsum = 1 + (kind == QS_Q2 ? 1 : (kind == QS_Q23 ? 2 : 4)), w = 2 * (1 + q.nq);
+  HM_TRY(ensure_host(c, (void **)&c->h_out, &c->h_out_cap, sizeof(double) * 2 * SLOT * (size_t)nitems + 64));
+  if (!c->d_ticket) {
+    HM_CUDA(c, cudaMalloc((void **)&c->d_ticket, 256));
+    HM_CUDA(c, cudaMemsetAsync(c->d_ticket, 0, 256, c->stream));
+  }
+  HM_CUDA(c, cudaEventRecord(c->ev0, c->stream));
+  const int rc = enqueue_sweeps(c, items, nitems, kind, qp, nsum, precision);
+  if (rc != HM_OK) {
+    // the sweeps queued before the failure still write to their slots, which the next call
+    // clears on the host
+    cudaStreamSynchronize(c->stream);
+    return rc;
+  }
   HM_CUDA(c, cudaStreamSynchronize(c->stream));
   float ms = 0.f;
   HM_CUDA(c, cudaEventElapsedTime(&ms, c->ev0, c->ev1));
