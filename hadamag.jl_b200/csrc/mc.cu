@@ -81,9 +81,11 @@ __global__ void __launch_bounds__(128) k_mc_p1(McArgs a) {
   p1_unit<R, HI, false>(src, xx, row, a.inter + (size_t)c * ((size_t)1 << (a.n - 1)), sm, lane);
 }
 
-// n >= 16, pass 2: warp units (chain, tile) -> part[chain][tile]
+// n >= 16, pass 2: warp units (chain, tile) -> part[chain][tile].  Three CTAs per SM: left to
+// itself the compiler gives the generic q 198 registers, which leaves two and idle time in the
+// powers (q = 2.7, us per step: n = 18, 13 chains 87 -> 63; n = 16, 201 chains 265 -> 213).
 template <int HI, int QS>
-__global__ void __launch_bounds__(128) k_mc_p2(McArgs a) {
+__global__ void __launch_bounds__(128, 3) k_mc_p2(McArgs a) {
   constexpr int R = 32, PB = 10;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
