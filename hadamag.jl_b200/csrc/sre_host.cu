@@ -4,6 +4,7 @@
 #include <math.h>
 
 #include <mutex>
+#include <algorithm>
 #include <vector>
 
 #include "sre_launch.cuh"
@@ -296,18 +297,21 @@ static __global__ void k_tune_state(double2 *psi, uint64_t len) {
   }
 }
 
-// Autotuner of the two-pass sweep of one (n, precision): times hm_sre_range on `sample`
-// Gray indices (starting at 1024, where the sweep's steady state begins) for
-//   the stage kernels with X = 1, 2, 4, ... X-strings per stage (ring up to 1 GiB), and
+// Autotuner of the sweep of one (n, precision): times q = 2 on `sample` Gray indices (starting
+// at 1024, where the sweep's steady state begins) for
+//   the stage kernels with the default batch, with batches of 1 .. 12 whole rounds over the
+//   GPU's warps, and of 1, 2, 4, ... X-strings and 1.25 and 1.5 times these (ring up to 1 GiB),
+//   or, where one CTA holds an X-string and there is no batch, that kernel; and
 //   the queue sweep with X = 1, 2, 4, ... X-strings per ring slot (4 slots up to 1 GiB)
-//   at full occupancy and at one CTA per SM,
-// keeps the fastest (kernel time, CUDA events) and records engine, batch size and CTAs per
-// SM for this (n, precision); later calls use them unless a knob forces another choice.
+//   at full occupancy and at one CTA per SM.
+// It records engine, batch size and CTAs per SM of the fastest (kernel time, CUDA events) for
+// this (n, precision); later calls use them unless a knob forces another choice.  The default
+// stays unless another choice is 1 % faster, about the spread between two timings.
 extern "C" int hm_autotune(hm_ctx *c, int n, int precision, int *best_x, double *best_us_per_x) {
   if (!c) return HM_ERR_ARG;
   c->err.clear();
   if (!best_x || !best_us_per_x) return hm::set_err(c, HM_ERR_ARG, "null output pointer");
-  if (n < 12 || n > 21) return hm::set_err(c, HM_ERR_SIZE, "autotune: n = %d outside the two-pass range [12, 21]", n);
+  if (n < 12 || n > 21) return hm::set_err(c, HM_ERR_SIZE, "autotune: n = %d outside [12, 21]", n);
   if (precision != HM_FP64 && precision != HM_FP32)
     return hm::set_err(c, HM_ERR_ARG, "autotune: precision must be HM_FP64 or HM_FP32");
   HM_CUDA(c, cudaSetDevice(c->device));
@@ -321,16 +325,18 @@ extern "C" int hm_autotune(hm_ctx *c, int n, int precision, int *best_x, double 
   const hm::QueueCfg qsaved = qc;
   const int pi = precision == HM_FP64 ? 0 : 1;
   const uint64_t per_x = (len / 2) * (precision == HM_FP64 ? sizeof(double2) : sizeof(float2));
-  const uint64_t rows = len / 2 / 1024;  // pass-1 units per X-string
-  // sample: at least 8 batches of the largest candidate and about 8192 pass-1 units
+  // sample: at least 8 batches of the largest candidate, and about 30 ms at the larger n, where a
+  // longer sweep's steady state decides: on samples of 2 to 4 ms the capture of the stage graph
+  // weighed as much as a bad batch (n = 19, FP64: X = 64 won and cost 1.97 us per X-string, the
+  // default 1.69)
   uint64_t xmax = 1;
   while (xmax < 256 && 2 * (xmax * 2) * per_x <= (1ull << 30)) xmax *= 2;
-  uint64_t sample = std::max<uint64_t>(8 * xmax, (8192 + rows - 1) / rows);
+  uint64_t sample = std::max<uint64_t>(8 * xmax, 1ull << (33 - n));
   if (1024 + sample > len) sample = len - 1024;
   hm::QReq q;
   q.nq = 1;
   q.q[0] = 2.0;
-  double dd[10], best = 1e300;
+  double dd[10], best = 1e300, bar = 1e300;
   int bx = 0, beng = 1, bcps = 0;
   int rc = HM_OK;
   auto timeit = [&](double *t) {
@@ -340,13 +346,28 @@ extern "C" int hm_autotune(hm_ctx *c, int n, int precision, int *best_x, double 
       if (rc == HM_OK && rep > 0) *t = std::min(*t, c->last_ms);
     }
   };
-  // stage kernels: every power of two up to xmax and the sizes 1.25 and 1.5 times one
-  // (the kernel decodes its units with a division, so any X works; at n = 20 in FP64
-  // X = 10 beats both 8 and 16)
+  auto better = [&](double t) {
+    if (rc != HM_OK || t >= bar) return false;
+    best = t;
+    bar = bar == 1e300 ? 0.99 * t : t;  // the first one is the default
+    return true;
+  };
   std::vector<uint64_t> xs;
-  for (uint64_t P = 1; P <= xmax; P *= 2)
-    for (uint64_t X : {P, P + P / 4, P + P / 2})
-      if (X <= xmax && (xs.empty() || X > xs.back())) xs.push_back(X);
+  const bool single = n <= hm::single_cta_max(precision == HM_FP64);
+  if (single) {
+    xs.push_back(1);  // no batch to choose
+  } else {
+    const bool stage = precision == HM_FP64 && hm::on_stage_kernel<double, hm::QS_Q2>(n);
+    for (uint64_t P = 1; P <= xmax; P *= 2)
+      for (uint64_t X : {P, P + P / 4, P + P / 2}) xs.push_back(X);
+    const uint64_t warps = (uint64_t)c->num_sms * (precision == HM_FP64 ? 8 : 16);
+    for (uint64_t m = 1; m <= 12; ++m) xs.push_back(m * warps >> (n - 10));
+    std::sort(xs.begin(), xs.end());
+    xs.erase(std::unique(xs.begin(), xs.end()), xs.end());
+    const uint64_t def = (uint64_t)hm::measured_x(precision == HM_FP64, n, stage);
+    xs.erase(std::remove_if(xs.begin(), xs.end(), [&](uint64_t X) { return X < 1 || X > xmax || X == def; }), xs.end());
+    xs.insert(xs.begin(), def);
+  }
   qc.engine = 1;
   for (size_t xi = 0; xi < xs.size() && rc == HM_OK; ++xi) {
     const uint64_t X = xs[xi];
@@ -355,8 +376,7 @@ extern "C" int hm_autotune(hm_ctx *c, int n, int precision, int *best_x, double 
     cfg.ring_mib = std::max<int>(saved.ring_mib, (int)((2 * X * per_x + (1 << 20) - 1) >> 20));
     double t;
     timeit(&t);
-    if (rc == HM_OK && t < best) {
-      best = t;
+    if (better(t)) {
       bx = (int)X;
       beng = 1;
       bcps = 0;
@@ -374,8 +394,7 @@ extern "C" int hm_autotune(hm_ctx *c, int n, int precision, int *best_x, double 
       qc.ctas_per_sm = cps;
       double t;
       timeit(&t);
-      if (rc == HM_OK && t < best) {
-        best = t;
+      if (better(t)) {
         bx = (int)X;
         beng = 2;
         bcps = cps;

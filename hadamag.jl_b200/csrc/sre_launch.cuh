@@ -1,5 +1,5 @@
-// sre_launch.cuh -- host launchers for the exact-SRE kernels (instantiated per precision
-// in sre_fp64.cu / sre_fp32.cu).
+// sre_launch.cuh -- host launchers for the exact-SRE kernels (instantiated per precision and
+// moment set in sre_fp64_q2.cu, sre_fp64_q23.cu, ...).
 #pragma once
 #include "hm_ctx.h"
 #include "sre_kernels.cuh"
@@ -7,6 +7,17 @@
 #include "sweep3.cuh"
 
 namespace hm {
+
+// The largest n whose X-strings one CTA holds (k_sre_wide); two passes from there up.
+constexpr int single_cta_max(bool fp64) { return fp64 ? 14 : 15; }
+
+// Two-pass sweeps that stay on k_sre_stage, FP64 (us per X-string on B200; the other side is
+// k_sre_wide_stage at its best batch): n = 20, q = 2 X = 10 3.74 (X = 7 3.87), q = 2 and 3 3.85
+// (q = 3 4.06); n = 19, q = 2 and 3 X = 16 1.84 (X = 9 1.89).  Both kernels are bound by the
+// ring's traffic there, and its tensor stores need no group of four.
+template <typename T, int QS> constexpr bool on_stage_kernel(int n) {
+  return sizeof(T) == 8 && ((n == 20 && QS != QS_GEN) || (n == 19 && QS == QS_Q23));
+}
 
 // Tunables of the two-pass stage kernels (set through hm_set_param): a batch holds about
 // `units_target` warp units per pass (X = units_target / 2^(n-11) X-strings, or X when set
@@ -19,21 +30,21 @@ namespace hm {
 //   FP64  n = 15: X = 148 (0.107; 74: 0.120)    n = 16: X = 111 (0.191; 74: 0.195, 37: 0.22)
 //         n = 17: X = 55 (0.377; 37: 0.387)     n = 18: X = 27 (0.784; 18: 0.785, 37: 0.796)
 //         n = 19: X = 9 (1.735; 14: 1.759, 4: 1.83)  n = 21: X = 4 (9.10; 3: 9.29, 2: 9.87)
+//         n = 20, generic q (bound by the powers): X = 10 (q = 4 4.94, q = 2.7 19.8; 7: 4.93, 22.3)
 //   FP32  n = 16: X = 148 (0.106; 74: 0.124)
 //         n = 17: X = 110 (0.197; 74: 0.204)    n = 18: X = 55 (0.403; 37: 0.413)
 //         n = 19: X = 18 (0.861; 28: 0.878)     n = 20: X = 9 (1.97; 7: 2.02)
 //         n = 21: X = 4 (4.65; 2: 4.90)
 // Against the rows and tiles of k_sre_stage, which ran every size before: FP64 0.116, 0.206,
 // 0.430, 0.852, 1.815, 3.79, 10.33 for n = 15 .. 21, FP32 0.115, 0.221, 0.446, 0.967, 2.70,
-// 10.02 for n = 16 .. 21.  FP64 at n = 20 stays with k_sre_stage (X = 10: 3.74, 3.83 before its q = 2
-// moments by quads; 3.87 here at X = 7): both are bound by the ring's traffic there, and its
-// tensor stores need no group of four.  So does FP64 at n = 19 for q = 2 and 3 together
-// (X = 16: 1.84; 1.89 here at X = 9).
+// 10.02 for n = 16 .. 21.
 // hm_autotune measures and records a batch for the machine at hand; setting
 // HM_PARAM_BATCH, _UNITS or _RING switches to the generic rule.
-inline int measured_x(bool fp64, int n) {
+inline int measured_x(bool fp64, int n, bool stage_kernel) {
   static const int f64[7] = {148, 111, 55, 27, 9, 10, 4}, f32[7] = {0, 148, 110, 55, 18, 9, 4};
-  return (n >= 15 && n <= 21) ? (fp64 ? f64 : f32)[n - 15] : 0;
+  if (n < 15 || n > 21) return 0;
+  if (stage_kernel) return n == 19 ? 16 : 10;
+  return (fp64 ? f64 : f32)[n - 15];
 }
 
 struct TwoPassCfg {
@@ -44,9 +55,14 @@ struct TwoPassCfg {
   int graph_stages = 128;  // stages per captured graph (128: 0.4 % faster than 32 at n = 20)
   int adj_x = 0;  // X-strings per batch of the adjoint stage kernels (0: the default rule)
   // batch sizes chosen by hm_autotune, per precision (0 FP64, 1 FP32) and qubit count;
-  // 0 = not tuned.  Used when HM_PARAM_BATCH is not set.
+  // 0 = not tuned.  Used when HM_PARAM_BATCH is not set (see tuned_batch).
   int tuned_x[2][32] = {};
 };
+// hm_autotune times q = 2: its batch is that of the kernel that runs q = 2 at this size, and
+// not of one that other moment sets run there
+template <typename T, int QS> inline int tuned_batch(const TwoPassCfg &cfg, int n) {
+  return on_stage_kernel<T, QS>(n) == on_stage_kernel<T, QS_Q2>(n) ? cfg.tuned_x[sizeof(T) == 8 ? 0 : 1][n] : 0;
+}
 
 TwoPassCfg &twopass_cfg();
 
@@ -94,7 +110,7 @@ static int launch_fused(hm_ctx *c, const SreArgs &a0, int *nwarps_out) {
   return HM_OK;
 }
 
-// n = 12, 13, 14: one CTA of G = 2^(n-11) warps per X-string (see k_sre_wide).  n = 14 is
+// n = 12, 13, 14 (FP64 also 11, FP32 15): one CTA of G = 2^(n-11) warps per X-string (see k_sre_wide).  n = 14 is
 // the last size whose planes (128 KB in FP64) and registers (8 warps of 255) fit an SM; the
 // two-pass sweep was half as fast at each of the three sizes (figures in sre_wide.cuh).
 template <typename T, int G, int QS>
@@ -195,8 +211,8 @@ static int launch_stages(hm_ctx *c, const SreArgs &a0, int *nwarps_out) {
   const TwoPassCfg def;
   const bool generic = cfg.X_set || cfg.units_target != def.units_target || cfg.ring_mib != def.ring_mib;
   uint64_t X, ring_mib = (uint64_t)cfg.ring_mib;
-  const int tuned = cfg.tuned_x[sizeof(T) == 8 ? 0 : 1][a.n];
-  const int measured = generic ? 0 : (a.n == 19 ? 16 : measured_x(sizeof(T) == 8, a.n));
+  const int tuned = tuned_batch<T, QS>(cfg, a.n);
+  const int measured = generic ? 0 : measured_x(sizeof(T) == 8, a.n, true);
   if (cfg.X_set) {
     X = (uint64_t)cfg.X;
   } else if (tuned > 0 || measured > 0) {
@@ -273,8 +289,8 @@ static int launch_wide_stages(hm_ctx *c, const SreArgs &a0, int *nwarps_out) {
   const TwoPassCfg def;
   const bool generic = cfg.X_set || cfg.units_target != def.units_target || cfg.ring_mib != def.ring_mib;
   uint64_t X, ring_mib = (uint64_t)cfg.ring_mib;
-  const int tuned = cfg.tuned_x[sizeof(T) == 8 ? 0 : 1][N];
-  const int measured = generic ? 0 : measured_x(sizeof(T) == 8, N);
+  const int tuned = tuned_batch<T, QS>(cfg, N);
+  const int measured = generic ? 0 : measured_x(sizeof(T) == 8, N, false);
   if (cfg.X_set) {
     X = (uint64_t)cfg.X;
   } else if (tuned > 0 || measured > 0) {
@@ -424,13 +440,13 @@ static int dispatch_sre(hm_ctx *c, const SreArgs &a, int *nw) {
         return launch_wide_stages<T, 17, QS>(c, a, nw);
       case 7:
         return launch_wide_stages<T, 18, QS>(c, a, nw);
-      case 8:  // FP64, q = 2 and 3: see measured_x
-        if constexpr (sizeof(T) == 8 && QS == QS_Q23)
+      case 8:
+        if constexpr (on_stage_kernel<T, QS>(19))
           return launch_stages<T, R, 8, QS>(c, a, nw);
         else
           return launch_wide_stages<T, 19, QS>(c, a, nw);
-      case 9:  // FP64, q = 2 (and 3): see measured_x
-        if constexpr (sizeof(T) == 8 && QS != QS_GEN)
+      case 9:
+        if constexpr (on_stage_kernel<T, QS>(20))
           return launch_stages<T, R, 9, QS>(c, a, nw);
         else
           return launch_wide_stages<T, 20, QS>(c, a, nw);

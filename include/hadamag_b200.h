@@ -65,14 +65,16 @@ const char *hm_last_error(hm_ctx *ctx);
  * stream).  Lets a caller time the kernels with events on that stream. */
 int hm_set_stream(hm_ctx *ctx, void *cuda_stream);
 
-/* Tuning knobs of the exact-SRE multi-pass sweeps (n >= 12); the autotuner sets them,
- * defaults apply otherwise.  HM_PARAM_BATCH: X-strings per batch (1..4096; the queue
- * sweep rounds it down to a power of two; 0 = derive it from HM_PARAM_UNITS);
+/* Tuning knobs of the exact-SRE multi-pass sweeps (n >= 15; FP32 16).  At n = 12, 13, 14 (FP32
+ * also 15) one CTA holds an X-string and there is no batch: there HM_PARAM_BATCH acts only on
+ * the queue sweep, the next three on nothing.  The autotuner sets a batch, defaults apply
+ * otherwise.  HM_PARAM_BATCH: X-strings per batch (1..4096; the queue sweep rounds it down
+ * to a power of two; 0 = the tuned or default batch);
  * HM_PARAM_RING: budget of the two-batch intermediate ring in MiB (8..4096; it should
  * stay L2 resident); HM_PARAM_UNITS: warp units per pass the automatic batch size aims
  * for (256..2^20); HM_PARAM_GRAPH: stage kernels captured per CUDA graph (1..1024,
  * default 128; sweeps of at most as many stages launch them directly); HM_PARAM_ADJ_BATCH:
- * X-strings per batch of hm_sre_grad's stage kernels (power of two, 1..1024).  Value 0
+ * X-strings per batch of hm_sre_grad's stage kernels, n >= 15 (power of two, 1..1024).  Value 0
  * restores the default.  Process-wide; returns HM_ERR_ARG for an unknown knob or value. */
 #define HM_PARAM_BATCH 1
 #define HM_PARAM_RING 2
@@ -107,14 +109,18 @@ int hm_set_stream(hm_ctx *ctx, void *cuda_stream);
 #define HM_PARAM_BATCH_SPLIT_N 14
 int hm_set_param(int param, int value);
 
-/* Autotuner of the two-pass sweep (no reference counterpart): times the sweep of an n-qubit
- * state on a sample of Gray indices with the stage kernels (X = 1, 2, 3, 4, 5, 6, 8, 10,
- * 12, ... X-strings per stage: each power of two and 1.25 and 1.5 times it) and with the
- * queue sweep (X = 1, 2, 4, ... X-strings per ring slot, at full
- * occupancy and at one CTA per SM), records the fastest engine, batch size and CTAs per
- * SM for this (n, precision) in a process-wide table that later calls use unless a knob
- * forces another choice, and returns the batch size with the measured microseconds per
- * X-string.  12 <= n <= 21, precision HM_FP64 or HM_FP32.  Takes a second or two. */
+/* Autotuner of the exact sweep (no reference counterpart): times q = 2 on a sample of Gray
+ * indices of an n-qubit state with the stage kernels (the default batch, batches of whole rounds
+ * over the GPU, and X = 1, 2, 3, 4, 5, 6, 8, 10, 12, ... X-strings per stage: each power of two
+ * and 1.25 and 1.5 times it) and with the queue sweep (X = 1, 2, 4, ... X-strings per ring
+ * slot, at full occupancy and at one CTA per SM), records the fastest engine, batch size and
+ * CTAs per SM for this (n, precision) in a process-wide table that later calls use unless a
+ * knob forces another choice, and returns the batch size with the measured microseconds per
+ * X-string.  Anything but the default has to be 1 % faster than it.  A batch is used by the
+ * moment sets that run the timed kernel (not by q = 2 and 3 together at n = 19 in FP64, nor by
+ * other q at n = 20).  Where one CTA holds an X-string (n = 12, 13, 14; FP32 also 15) the stage
+ * engine has no batch, and the batch size returned for it is 1.  12 <= n <= 21, precision
+ * HM_FP64 or HM_FP32.  Takes a few seconds. */
 int hm_autotune(hm_ctx *ctx, int n, int precision, int *best_x, double *best_us_per_x);
 
 /* The choice hm_autotune recorded for (n, precision): engine 0 (not tuned), 1 (stage
