@@ -30,7 +30,7 @@ template <typename T, int QS> constexpr bool on_stage_kernel(int n) {
 //   FP64  n = 15: X = 148 (0.107; 74: 0.120)    n = 16: X = 111 (0.191; 74: 0.195, 37: 0.22)
 //         n = 17: X = 55 (0.377; 37: 0.387)     n = 18: X = 27 (0.784; 18: 0.785, 37: 0.796)
 //         n = 19: X = 9 (1.735; 14: 1.759, 4: 1.83)  n = 21: X = 4 (9.10; 3: 9.29, 2: 9.87)
-//         n = 20, generic q (bound by the powers): X = 10 (q = 4 4.94, q = 2.7 19.8; 7: 4.93, 22.3)
+//         n = 20, q other than 2, 3: X = 9 (q = 4 4.46, q = 2.7 18.3; 7: 4.40, 21.7; 10: 4.60, 19.3)
 //   FP32  n = 16: X = 148 (0.106; 74: 0.124)
 //         n = 17: X = 110 (0.197; 74: 0.204)    n = 18: X = 55 (0.403; 37: 0.413)
 //         n = 19: X = 18 (0.861; 28: 0.878)     n = 20: X = 9 (1.97; 7: 2.02)
@@ -41,7 +41,7 @@ template <typename T, int QS> constexpr bool on_stage_kernel(int n) {
 // hm_autotune measures and records a batch for the machine at hand; setting
 // HM_PARAM_BATCH, _UNITS or _RING switches to the generic rule.
 inline int measured_x(bool fp64, int n, bool stage_kernel) {
-  static const int f64[7] = {148, 111, 55, 27, 9, 10, 4}, f32[7] = {0, 148, 110, 55, 18, 9, 4};
+  static const int f64[7] = {148, 111, 55, 27, 9, 9, 4}, f32[7] = {0, 148, 110, 55, 18, 9, 4};
   if (n < 15 || n > 21) return 0;
   if (stage_kernel) return n == 19 ? 16 : 10;
   return (fp64 ? f64 : f32)[n - 15];

@@ -24,3 +24,14 @@ def test_direct_launches_and_replays_agree(ctx, hm, n, qs):
         N.set_param(N.HM_PARAM_BATCH, 0)
         N.set_param(N.HM_PARAM_GRAPH, 0)
     assert np.array_equal(direct[0], replay[0]) and np.array_equal(direct[1], replay[1])
+
+
+def test_default_batch_belongs_to_the_kernel(ctx, hm):
+    """At n = 20 in FP64 q = 2 and other q run different kernels, whose default batches are 10 and
+    9: 90 X-strings take 9 and 10 batches, one stage more, and the fold."""
+    psi = rand_state(1 << 20, 170)
+    counts = []
+    for qs in ((2.0,), (4.0,)):
+        ctx.sre_range(psi, 2000, 2090, qs, hm.HM_FP64)
+        counts.append(ctx.last_launch_count())
+    assert counts == [11, 12]
