@@ -132,12 +132,13 @@ static int launch_wide(hm_ctx *c, const SreArgs &a0, int *nwarps_out) {
   return HM_OK;
 }
 
-// Launch the nst chained stage kernels of a sweep (node s runs stage s).  Up to G stages, one
-// graph's worth, go out as direct launches: a stage runs longer than its launch takes (about
+// Launch the nst chained stage kernels of a sweep (node s runs stage s).  Up to 2 G stages, two
+// graphs' worth, go out as direct launches: a stage runs longer than its launch takes (about
 // 2 us), while capturing and instantiating a graph holds back the first stage by about 3 us a
-// node (B200, whole call: n = 19, 36 stages 1206 -> 1037 us, 89 stages 2098 -> 1841; n = 15, 87
-// stages 1521 -> 1313.  Under a bound of 32 stages, ranges that once fitted into 32 of the
-// larger batches of that time, at n = 18 and 19, had become 7 to 14 % slower).  Longer sweeps
+// node, and the last replay runs up to G - 1 stages without a batch (B200: n = 19, 36 stages
+// 1206 -> 1037 us per call, 129 stages 2439 -> 1985 us of kernels).  Under a bound of 32
+// stages, ranges that the larger batches of that time ran in 32 to 100 stages had become 5
+// to 14 % slower at n = 18 and 19.  Longer sweeps
 // replay a captured graph of G stages, with a one-thread kernel advancing the stage base in
 // device memory after every replay.
 template <typename Kern, typename Args>
@@ -158,7 +159,7 @@ static int run_stage_chain(hm_ctx *c, Kern kern, Args &a, int nst, int blocks, i
     return cudaLaunchKernelEx(&lc, kern, a);
   };
   cudaError_t ce = cudaSuccess;
-  if (nst <= G) {
+  if (nst <= 2 * G) {
     for (int s = 0; s < nst && ce == cudaSuccess; ++s) ce = launch(s);
     c->launches += nst;
     if (ce != cudaSuccess) return set_err(c, HM_ERR_CUDA, "%s launch failed: %s", what, cudaGetErrorString(ce));

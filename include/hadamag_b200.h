@@ -73,7 +73,7 @@ int hm_set_stream(hm_ctx *ctx, void *cuda_stream);
  * HM_PARAM_RING: budget of the two-batch intermediate ring in MiB (8..4096; it should
  * stay L2 resident); HM_PARAM_UNITS: warp units per pass the automatic batch size aims
  * for (256..2^20); HM_PARAM_GRAPH: stage kernels captured per CUDA graph (1..1024,
- * default 128; sweeps of at most as many stages launch them directly); HM_PARAM_ADJ_BATCH:
+ * default 128; sweeps of at most twice as many stages launch them directly); HM_PARAM_ADJ_BATCH:
  * X-strings per batch of hm_sre_grad's stage kernels, n >= 15 (power of two, 1..1024).  Value 0
  * restores the default.  Process-wide; returns HM_ERR_ARG for an unknown knob or value. */
 #define HM_PARAM_BATCH 1
