@@ -242,8 +242,12 @@ struct QParams {
   int direct;  // one q, an integer or a half-integer (half_integer_q)
 };
 
-// (F^2)^q with 2q an integer is F^2 to an integer power, times |F| if 2q is odd
-__host__ __device__ inline bool half_integer_q(double q) { return 2.0 * q == floor(2.0 * q) && q >= 1.0 && q <= 16.0; }
+// (F^2)^q with 2q an integer is |F| to an integer power.  q = 8.5 is left to pow(): its four
+// squarings in a row, each doubling the error before it, end above pow's (rms 4.4e-16 of a value
+// against 4.0e-16; 0.77 to 1.0 times the errors of squaring F^2 and of pow at all other q).
+__host__ __device__ inline bool half_integer_q(double q) {
+  return 2.0 * q == floor(2.0 * q) && q >= 1.0 && q <= 16.0 && q != 8.5;
+}
 
 inline void set_qparams(QParams &qp, const double *q, int nq) {
   qp.nq = nq;
@@ -254,26 +258,37 @@ inline void set_qparams(QParams &qp, const double *q, int nq) {
   }
 }
 
-// y^q and |f| y^(q - 1/2) for y = f^2, half_integer_q(q), N values side by side: the bits of
-// the exponent from the second one down, square and multiply.
+// r = f^2 -> |f|^(2q), half_integer_q(q), N values side by side: the bits of the exponent 2q
+// from the second one down, square and multiply by f, which has no rounding of its own.
 template <int N>
-__device__ __forceinline__ void pow_half(const double (&f)[N], const double (&y)[N], double q, double (&r)[N]) {
-  const int e2 = (int)(2.0 * q), e = e2 >> 1;
-#pragma unroll
-  for (int t = 0; t < N; ++t) r[t] = y[t];
+__device__ __forceinline__ void pow_half(const double (&f)[N], double (&r)[N], double q) {
+  const int e = (int)(2.0 * q);
+  int b = 30 - __clz(e);
 #pragma unroll 1
-  for (int b = 30 - __clz(e); b >= 0; --b) {
-#pragma unroll
-    for (int t = 0; t < N; ++t) r[t] *= r[t];
+  while (true) {
     if ((e >> b) & 1) {
 #pragma unroll
-      for (int t = 0; t < N; ++t) r[t] *= y[t];
+      for (int t = 0; t < N; ++t) r[t] *= f[t];
     }
-  }
-  if (e2 & 1) {
+    if (--b < 0) break;
 #pragma unroll
-    for (int t = 0; t < N; ++t) r[t] *= fabs(f[t]);
+    for (int t = 0; t < N; ++t) r[t] *= r[t];
   }
+  if (e & 1) {
+#pragma unroll
+    for (int t = 0; t < N; ++t) r[t] = fabs(r[t]);
+  }
+}
+
+template <int N> __device__ __forceinline__ double tree_sum(const double (&v)[N]) {
+  double s[N];
+#pragma unroll
+  for (int t = 0; t < N; ++t) s[t] = v[t];
+#pragma unroll
+  for (int w = N / 2; w > 0; w >>= 1)
+#pragma unroll
+    for (int t = 0; t < w; ++t) s[t] += s[t + w];
+  return s[0];
 }
 
 // Generic Renyi indices, per-lane sums of F^2 and (F^2)^q of the R complex registers.
@@ -281,7 +296,9 @@ __device__ __forceinline__ void pow_half(const double (&f)[N], const double (&y)
 //     its 128 registers), so that the powers are independent chains over the FP64 latency; the
 //     exponent is uniform over the grid.  A step of the loop over its bits is one product per
 //     value.  FP64 on B200, all 2^n X-strings: n = 13 q = 4 318 -> 155 us (staged, four chains),
-//     q = 2.5 1.50 ms -> 155 us (pow); n = 11 q = 4 52 -> 33 us; n = 20 q = 4 7.2 -> 5.0 us each.
+//     q = 2.5 1.50 ms -> 155 us (pow); n = 11 q = 4 52 -> 33 us; n = 20 q = 4 7.2 -> 4.5 us each.
+//     FP32, us per X-string, staged -> this: n = 13 q = 4 0.053 -> 0.014, n = 18 1.53 -> 0.58, n = 20
+//     7.2 -> 2.6, n = 22 45 -> 29, n = 24 162 -> 134.  F^2 is summed before it is raised, in place.
 //     Error of the sums against extended precision, n = 6 .. 11: 7e-16 at q = 2.5 (pow 13e-16).
 //     (A list of several q would keep all values and the sums in registers, which spill.)
 template <int R, typename V>
@@ -290,22 +307,15 @@ __device__ __forceinline__ void lane_moments_direct(const V (&v)[R], double *s, 
   double a2 = 0.0, ag = 0.0;
 #pragma unroll
   for (int c = 0; c < 2 * R / N; ++c) {
-    double f[N], y[N], r[N];
+    double f[N], r[N];
 #pragma unroll
     for (int t = 0; t < N; ++t) {
       f[t] = (double)(t & 1 ? v[(c * N + t) / 2].y : v[(c * N + t) / 2].x);
-      y[t] = f[t] * f[t];
+      r[t] = f[t] * f[t];
     }
-    pow_half(f, y, qp.q[0], r);
-#pragma unroll
-    for (int w = N / 2; w > 0; w >>= 1)
-#pragma unroll
-      for (int t = 0; t < w; ++t) {
-        y[t] += y[t + w];
-        r[t] += r[t + w];
-      }
-    a2 += y[0];
-    ag += r[0];
+    a2 += tree_sum(r);
+    pow_half(f, r, qp.q[0]);
+    ag += tree_sum(r);
   }
   s[0] = a2;
   s[1] = ag;
@@ -331,7 +341,9 @@ __device__ __noinline__ void lane_moments_gen(const T *sm, int lane, double *s, 
     for (int k = 0; k < qp.nq; ++k) {
       const double q = qp.q[k];
       if (half_integer_q(q)) {
-        pow_half(f, y, q, r);
+#pragma unroll
+        for (int t = 0; t < 4; ++t) r[t] = y[t];
+        pow_half(f, r, q);
       } else {
 #pragma unroll
         for (int t = 0; t < 4; ++t) r[t] = pow(y[t], q);
