@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(128) k_adj_p1(AdjArgs a) {
     xi_.jt = a.n - 1;
   }
   const double2 *src = xi_.sw < 0 ? a.psi : a.psi_sw[xi_.sw];
-  p1_unit<R, HI, false>(src, xi_, rho, ring, sm, lane);
+  p1_unit<R, HI>(src, xi_, rho, ring, sm, lane);
 }
 
 // Pass 2: forward high bits, pointwise map, backward high bits, in place
@@ -777,7 +777,7 @@ __global__ void __launch_bounds__(ADJ_WARPS * 32, 2) k_adjs_p1(AdjStageArgs a) {
     xi.sw = -1;
     xi.xt = x;
     xi.jt = 63 - __clzll((long long)x);
-    p1_unit<R, HI, false>(a.psi, xi, rho, a.ring + ((size_t)(t % 3) * a.X + xs) * xlen, sm, lane, pre);
+    p1_unit<R, HI>(a.psi, xi, rho, a.ring + ((size_t)(t % 3) * a.X + xs) * xlen, sm, lane, pre);
   }
   wait_prior_grid();  // every CTA waits before it exits (transitive ordering of the chain)
 }

@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(128) k_mc_p1(McArgs a) {
     xx.jt = a.n - 1;
   }
   const double2 *src = xx.sw < 0 ? a.psi : a.psi_sw[xx.sw];
-  p1_unit<R, HI, false>(src, xx, row, a.inter + (size_t)c * ((size_t)1 << (a.n - 1)), sm, lane);
+  p1_unit<R, HI>(src, xx, row, a.inter + (size_t)c * ((size_t)1 << (a.n - 1)), sm, lane);
 }
 
 // n >= 16, pass 2: warp units (chain, tile) -> part[chain][tile].  Three CTAs per SM: left to

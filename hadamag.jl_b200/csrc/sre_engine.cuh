@@ -512,31 +512,10 @@ __device__ __forceinline__ XInfo make_xinfo(uint64_t k, uint64_t k_end, int n, i
   return xi;
 }
 
-// Pass 1: gather + build row rho of the (n-1)-bit index of x and transform its low PB
-// bits.  The conj side a = psi(row rH) is loaded straight into the registers that will
-// hold f; the partner row b = psi(row sH) goes to the warp's shared buffer through
-// cp.async (no registers held while in flight), is read back permuted by the low bits
-// of x, and the buffer is then reused for the transpose.
-__device__ __forceinline__ void cp_async16(void *smem_dst, const void *gmem_src) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem_src) : "memory");
-}
-__device__ __forceinline__ void cp_async8(void *smem_dst, const void *gmem_src) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(s), "l"(gmem_src) : "memory");
-}
-template <typename V>
-__device__ __forceinline__ void cp_async_v(V *smem_dst, const V *gmem_src) {
-  if constexpr (sizeof(V) == 16)
-    cp_async16(smem_dst, gmem_src);
-  else
-    cp_async8(smem_dst, gmem_src);
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-template <int R, bool STAGE_B, typename V>
-__device__ __forceinline__ void p1_build(V (&v)[R], const V *__restrict__ psi, const XInfo &xi, uint64_t rho, V *sm,
-                                         int lane) {
+// Pass 1: gather + build row rho of the (n-1)-bit index of x; its low PB bits are transformed
+// next (p1_unit, p1_unit_tma).
+template <int R, typename V>
+__device__ __forceinline__ void p1_build(V (&v)[R], const V *__restrict__ psi, const XInfo &xi, uint64_t rho, int lane) {
   constexpr int PB = ilog2c(R) + 5;
   if (xi.zero) {
     // x = 0: f(r) = |psi(r)|^2 paired on the top bit (jt = n - 1),
@@ -555,25 +534,11 @@ __device__ __forceinline__ void p1_build(V (&v)[R], const V *__restrict__ psi, c
   const uint32_t xL = (uint32_t)(xi.xt & ((1ull << PB) - 1ull));
   const V *rowA = psi + (rH << PB);
   const V *rowB = psi + (sH << PB);
-  if constexpr (STAGE_B) {
-    // partner row, in natural order, into the shared buffer
+  // both rows straight into registers (the partner permuted by the low bits of x)
 #pragma unroll
-    for (int i = 0; i < R; ++i) cp_async_v(sm + i * 32 + lane, rowB + i * 32 + lane);
-    // conj side straight into registers
-#pragma unroll
-    for (int i = 0; i < R; ++i) v[i] = ld_psi(rowA + i * 32 + lane);
-    cp_async_wait_all();
-    __syncwarp();
-#pragma unroll
-    for (int i = 0; i < R; ++i) v[i] = conj_mul(v[i], sm[(uint32_t)(i * 32 + lane) ^ xL]);
-    __syncwarp();  // the buffer is rewritten by the transpose
-  } else {
-    // both rows straight into registers (the partner permuted by the low bits of x)
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-      const uint32_t e = (uint32_t)(i * 32 + lane);
-      v[i] = conj_mul(ld_psi(rowA + e), ld_psi(rowB + (e ^ xL)));
-    }
+  for (int i = 0; i < R; ++i) {
+    const uint32_t e = (uint32_t)(i * 32 + lane);
+    v[i] = conj_mul(ld_psi(rowA + e), ld_psi(rowB + (e ^ xL)));
   }
 }
 
@@ -587,12 +552,12 @@ struct NoHook {
   __device__ __forceinline__ void operator()() const {}
 };
 
-template <int R, int HI, bool STAGE_B, typename V, typename Pre = NoHook>
+template <int R, int HI, typename V, typename Pre = NoHook>
 __device__ __forceinline__ void p1_unit(const V *__restrict__ psi, const XInfo &xi, uint64_t rho,
                                         V *__restrict__ inter_x, V *sm, int lane, const Pre &pre = Pre()) {
   constexpr int LOGR = ilog2c(R), PB = LOGR + 5, LOGC = PB - HI;
   V v[R];
-  p1_build<R, STAGE_B>(v, psi, xi, rho, sm, lane);
+  p1_build(v, psi, xi, rho, lane);
   reg_wht<R, 0, LOGR>(v);  // element bits 5 .. PB-1
   transpose_ab<R>(v, sm, lane);
   reg_wht<R, 0, 5>(v);  // element bits 0 .. 4
@@ -648,7 +613,7 @@ __device__ __forceinline__ void p1_unit_tma(const V *__restrict__ psi, const XIn
                                             const Pre &pre = Pre(), const Ready &ready = Ready()) {
   constexpr int LOGR = ilog2c(R);
   V v[R];
-  p1_build<R, false>(v, psi, xi, rho, sm, lane);  // registers only (no shared memory)
+  p1_build(v, psi, xi, rho, lane);  // registers only (no shared memory)
 #ifdef HM_TMEM_EXCHANGE
   reg_wht<R, 0, LOGR>(v);
   ready();  // the shared buffer is free from here on

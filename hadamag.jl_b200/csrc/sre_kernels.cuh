@@ -262,15 +262,15 @@ __global__ void __launch_bounds__(SRE_WARPS * 32, StageOcc<T>::value)
       if (a.tma)
         p1_unit_tma<R, HI, TM>(src, xi, sub, sm, lane, &a.tmap, a.g, (int)((b & 1) * a.X + xs), ta, pre, ready);
       else
-        p1_unit<R, HI, false>(src, xi, sub, inter_x, sm, lane, pre);
+        p1_unit<R, HI>(src, xi, sub, inter_x, sm, lane, pre);
     } else {
       double s[NQ + 1];
       wait_prior_grid();
       p2_unit<R, HI, QS, TM>(inter_x + (sub << PB), sm, lane, s, a.qp, ta, ready);
-      // The tile is dead once read (its slot is rewritten by pass 1 two stages later, in
-      // another launch): drop its L2 lines without writing them back to DRAM.  The next
-      // write to the slot comes after griddepcontrol.wait on the launch in between, which
-      // returns once this launch has finished and its memory operations are performed.
+      // The tile is dead once read (its slot is rewritten by pass 1 of the next stage, another
+      // launch): drop its L2 lines without writing them back to DRAM.  That write comes after
+      // the next launch's griddepcontrol.wait on this one, which returns once this launch
+      // has finished and its memory operations are performed.
       // Within one launch a discard is NOT ordered by release/acquire on B200: the queue
       // sweep, whose slots are rewritten inside the same launch, lost data when it
       // discarded its tiles, so it does not.

@@ -147,18 +147,18 @@ __device__ __forceinline__ void wide_moments(V (&v)[32], double *s, const QParam
     for (int c = 0; c < 4; ++c) {
       wht_class<0, TOP>(v, c);
 #pragma unroll
-    for (int i = TOP >= 2 ? c : 8 * c; i < (TOP >= 2 ? 32 : 8 * c + 8); i += (TOP >= 2 ? 4 : 1)) {
-      if constexpr (PAIR) {
-        if ((i >> TOP) & 1) continue;
-        const int k = i | (1 << TOP);
-        quad.add(i & 1, v[i].x, v[i].y, v[k].x, v[k].y);
-      } else {
-        if ((i >> TOP) & 3) continue;
-        const int k = i | (1 << TOP), m = i | (2 << TOP);
-        quad.add(0, v[i].x, v[k].x, v[m].x, v[m | k].x);
-        quad.add(1, v[i].y, v[k].y, v[m].y, v[m | k].y);
+      for (int i = TOP >= 2 ? c : 8 * c; i < (TOP >= 2 ? 32 : 8 * c + 8); i += (TOP >= 2 ? 4 : 1)) {
+        if constexpr (PAIR) {
+          if ((i >> TOP) & 1) continue;
+          const int k = i | (1 << TOP);
+          quad.add(i & 1, v[i].x, v[i].y, v[k].x, v[k].y);
+        } else {
+          if ((i >> TOP) & 3) continue;
+          const int k = i | (1 << TOP), m = i | (2 << TOP);
+          quad.add(0, v[i].x, v[k].x, v[m].x, v[m | k].x);
+          quad.add(1, v[i].y, v[k].y, v[m].y, v[m | k].y);
+        }
       }
-    }
     }
     quad.get(s);
   } else {
@@ -394,9 +394,8 @@ __global__ void __launch_bounds__(32 * WideCta<G>::WARPS, (sizeof(T) == 8 ? 8 : 
 #pragma unroll
         for (int q = 0; q <= NQ; ++q) dd_add(acc[q], s[q]);
       }
-      // The columns are dead once read (their slot is rewritten two stages later, after
-      // griddepcontrol.wait on the launch in between): drop their L2 lines without writing
-      // them back.
+      // The columns are dead once read (pass 1 of the next stage rewrites their slot, after its
+      // griddepcontrol.wait on this launch): drop their L2 lines without writing them back.
       constexpr uint32_t LPR = CHUNK * UPI / 128;  // lines per row
       const T *line = inter + ((size_t)((sub * G + w) * UPI) << (11 - HI));
       __syncwarp();  // every lane's reads come before

@@ -97,7 +97,7 @@ __device__ __forceinline__ void p1_unit3(const V *__restrict__ psi, const V *__r
     }
   } else {
     const XInfo xi = make_xinfo(k, k_end, n, PB);
-    p1_build<R, false>(v, src, xi, rho, sm, lane);  // registers only
+    p1_build(v, src, xi, rho, lane);  // registers only
   }
   reg_wht<R, 0, LOGR>(v);
   ready();
