@@ -295,8 +295,8 @@ template <int N> __device__ __forceinline__ double tree_sum(const double (&v)[N]
 //   one half-integer q (qp.direct): from the registers, 16 values at a time (FP32: 8, for
 //     its 128 registers), so that the powers are independent chains over the FP64 latency; the
 //     exponent is uniform over the grid.  A step of the loop over its bits is one product per
-//     value.  FP64 on B200, all 2^n X-strings: n = 13 q = 4 318 -> 155 us (staged, four chains),
-//     q = 2.5 1.50 ms -> 155 us (pow); n = 11 q = 4 52 -> 33 us; n = 20 q = 4 7.2 -> 4.5 us each.
+//     value.  FP64 on B200, all 2^n X-strings: n = 13 q = 4 318 -> 149 us (staged, four chains),
+//     q = 2.5 1.50 ms -> 151 us (pow); n = 11 q = 4 52 -> 27 us; n = 20 q = 4 7.2 -> 4.5 us each.
 //     FP32, us per X-string, staged -> this: n = 13 q = 4 0.053 -> 0.014, n = 18 1.53 -> 0.58, n = 20
 //     7.2 -> 2.6, n = 22 45 -> 29, n = 24 162 -> 134.  F^2 is summed before it is raised, in place.
 //     Error of the sums against extended precision, n = 6 .. 11: 7e-16 at q = 2.5 (pow 13e-16).

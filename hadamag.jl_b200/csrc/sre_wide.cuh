@@ -19,7 +19,7 @@
 //   q = 2   FP64  n = 12: 69 -> 31   n = 13: 226 -> 124   n = 14: 1107 -> 530
 //           FP32  n = 12: 60 -> 32   n = 13: 144 -> 81    n = 14: 614 -> 308
 //                 n = 15: 2180 -> 1430 (2030 with the two-pass sweep below)
-//   n = 13, FP64: q = 2 and 3 231 -> 136, q = 4 724 -> 155, q = 2.5 1498 -> 155
+//   n = 13, FP64: q = 2 and 3 231 -> 136, q = 4 724 -> 149, q = 2.5 1498 -> 151
 // FP64 at n = 13 is 1.04 clocks per complex element and SM, 0.55 of them FP64 issue.
 #pragma once
 #include "sre_kernels.cuh"
