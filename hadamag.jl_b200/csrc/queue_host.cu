@@ -110,16 +110,23 @@ int run_queue(hm_ctx *c, const QueueItem *items, int nitems, const QReq &q, int 
     return cx > cy;
   });
   // ring slot: X-strings of the largest two-pass state per batch from the tuned table or
-  // the default slot size
+  // the default slot size, but no more than some state of this launch fills (x = 0 of many
+  // states: one X-string of the largest)
   int nmax = 0;
+  long long fill = 0;
   for (int i = 0; i < nitems; ++i)
-    if (items[i].n >= 12 && items[i].ke > items[i].kb) nmax = std::max(nmax, items[i].n);
+    if (items[i].n >= 12 && items[i].ke > items[i].kb) {
+      nmax = std::max(nmax, items[i].n);
+      long long x = 1;
+      while (x < (long long)(items[i].ke - items[i].kb)) x <<= 1;
+      fill = std::max(fill, x << (items[i].n - 1));
+    }
   long long slot_elems = 0;
   if (nmax > 0) {
     int X = cfg.X_set ? cfg.X : cfg.tuned_x[fp64 ? 0 : 1][nmax];
     if (X <= 0) X = (int)std::max<long long>(1, ((long long)cfg.slot_mib << 20) / ((long long)vbytes << (nmax - 1)));
     while (X & (X - 1)) X &= X - 1;  // a power of two
-    slot_elems = (long long)X << (nmax - 1);
+    slot_elems = std::min((long long)X << (nmax - 1), fill);
   }
   const int K = std::max(cfg.K, cfg.lead + 1);
   const int cps = cfg.ctas_per_sm > 0 ? cfg.ctas_per_sm : (nmax > 0 ? cfg.tuned_cps[fp64 ? 0 : 1][nmax] : 0);
